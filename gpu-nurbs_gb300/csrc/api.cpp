@@ -251,13 +251,11 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
   s->basis_u = d.basis_u;
   s->basis_v = d.basis_v;
   e = cudaMemcpyAsync(A, img.data(), S.in_bytes, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = launch_basis(d.knots_u, p, d.knot_u, d.ns_u, s->basis_u, st);
-  if (e == cudaSuccess) e = launch_basis(d.knots_v, q, d.knot_v, d.ns_v, s->basis_v, st);
+  if (e == cudaSuccess)
+    e = launch_basis_pair(d.knots_u, p, d.knot_u, d.ns_u, s->basis_u, d.knots_v, q, d.knot_v, d.ns_v, s->basis_v, st);
   if (e == cudaSuccess) e = launch_span_matrices(d, s->basis_u, s->basis_v, (double*)d.m64, (float*)d.m32, st);
-  if (e == cudaSuccess) e = launch_tree(d, st);
+  if (e == cudaSuccess) e = launch_nodes(d, st);
   if (e == cudaSuccess) e = launch_centre_ders(d, st);
-  if (e == cudaSuccess) e = launch_cones(d, st);
-  if (e == cudaSuccess) e = launch_quadtree_boxes(d, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // img must outlive the copy
   if (e != cudaSuccess) {
     cudaFree(s->arena);
@@ -335,8 +333,9 @@ int nurbs_get_matrix_n_raw(double* matrix_n_dev, int p, int q, int nu, int nv, c
   d.weights = weights_dev;
   cudaError_t e = cudaMemcpyAsync(tmp + o_iu, iu.data(), nsu * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(tmp + o_iv, iv.data(), nsv * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = launch_basis(knots_u_dev, p, d.knot_u, nsu, (double*)(tmp + o_bu), st);
-  if (e == cudaSuccess) e = launch_basis(knots_v_dev, q, d.knot_v, nsv, (double*)(tmp + o_bv), st);
+  if (e == cudaSuccess)
+    e = launch_basis_pair(knots_u_dev, p, d.knot_u, nsu, (double*)(tmp + o_bu), knots_v_dev, q, d.knot_v, nsv,
+                          (double*)(tmp + o_bv), st);
   if (e == cudaSuccess)
     e = launch_span_matrices(d, (double*)(tmp + o_bu), (double*)(tmp + o_bv), matrix_n_dev, nullptr, st);
   // the host vectors above must outlive the async copies
@@ -402,10 +401,8 @@ int nurbs_build_tree(nurbs_surface_t s, int levels, void* stream) {
   if (!s) return fail(NURBS_E_INVALID, "NULL surface");
   if (levels != 2) return fail(NURBS_E_UNSUPPORTED, "only the 2-level tree is supported (got %d)", levels);
   cudaStream_t st = (cudaStream_t)stream;
-  CUDA_TRY(launch_tree(s->dev, st), "tree launch");
+  CUDA_TRY(launch_nodes(s->dev, st), "tree launch");
   CUDA_TRY(launch_centre_ders(s->dev, st), "seed-centre derivatives");
-  CUDA_TRY(launch_cones(s->dev, st), "normal cones");
-  CUDA_TRY(launch_quadtree_boxes(s->dev, st), "quadtree boxes");
   CUDA_TRY(cudaStreamSynchronize(st), "tree sync");
   s->tree_built = true;
   return NURBS_OK;

@@ -115,7 +115,6 @@ __device__ __forceinline__ void put_node(double* o, double a, double b, double c
 // code = base(d) + a * 2^d + b; base = 0, 1, 5), written when the surface is converted.  Deeper
 // nodes, and the halves of U / V splits, scan their control points.
 constexpr int kQtDepth = 3;
-constexpr int kQtBoxes = 1 + 4 + 16;
 __device__ __forceinline__ int code_depth(int c) { return c == 0 ? 0 : (c < 5 ? 1 : 2); }
 __device__ __forceinline__ int child_code(int pc, int hu, int hv) {
   if (pc < 0) return -1;
@@ -142,39 +141,6 @@ __device__ void node_box(const SurfDev& s, const double* nd, int t, int stride, 
     for (int c = 0; c < 3; ++c) {
       mn[c] = mn[c] > x[c] ? x[c] : mn[c];
       mx[c] = mx[c] < x[c] ? x[c] : mx[c];
-    }
-  }
-}
-
-// One CTA per precomputed box: the node's rectangle by the same midpoint splits as the search.
-__global__ void __launch_bounds__(256) k_quadtree_boxes(SurfDev s, double* __restrict__ qtbox) {
-  const int code = blockIdx.x;
-  const int d = code_depth(code), side = 1 << d, idx = code - (d == 0 ? 0 : (d == 1 ? 1 : 5));
-  const int a = idx / side, b = idx % side;
-  double nd[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
-  for (int l = d - 1; l >= 0; --l) {
-    const int hu = (a >> l) & 1, hv = (b >> l) & 1;
-    const double mu = (nd[0] + nd[2]) / 2, mv = (nd[1] + nd[3]) / 2;
-    if (hu) nd[0] = mu; else nd[2] = mu;
-    if (hv) nd[1] = mv; else nd[3] = mv;
-  }
-  double mn[3], mx[3];
-  node_box(s, nd, threadIdx.x, blockDim.x, mn, mx);
-  __shared__ double red[256][6];
-  for (int c = 0; c < 3; ++c) {
-    red[threadIdx.x][c] = mn[c];
-    red[threadIdx.x][3 + c] = mx[c];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int j = 1; j < (int)blockDim.x; ++j)
-      for (int c = 0; c < 3; ++c) {
-        mn[c] = fmin(mn[c], red[j][c]);
-        mx[c] = fmax(mx[c], red[j][3 + c]);
-      }
-    for (int c = 0; c < 3; ++c) {
-      qtbox[6 * code + c] = mn[c];
-      qtbox[6 * code + 3 + c] = mx[c];
     }
   }
 }
@@ -464,11 +430,6 @@ cudaError_t launch_quadtree_pq(const SurfDev& s, const double* P_, int64_t n, do
 }
 
 }  // namespace
-
-cudaError_t launch_quadtree_boxes(const SurfDev& s, cudaStream_t st) {
-  k_quadtree_boxes<<<kQtBoxes, 256, 0, st>>>(s, s.qtbox);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_invert_quadtree(const SurfDev& s, const double* P, int64_t n, double max_edge, double* uv,
                                    int* status, double* residual, int precision, unsigned* counter, cudaStream_t st) {

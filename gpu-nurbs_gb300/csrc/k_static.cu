@@ -157,8 +157,7 @@ extern "C" int nurbs_get_matrix_n_noalloc(double* matrix_n_dev, int p, int q, in
   d.knot_v = idx_v;
   d.cps = control_points_dev;
   d.weights = weights_dev;
-  e = launch_basis(knots_u_dev, p, idx_u, h.ns_u, bas_u, st);
-  if (e == cudaSuccess) e = launch_basis(knots_v_dev, q, idx_v, h.ns_v, bas_v, st);
+  e = launch_basis_pair(knots_u_dev, p, idx_u, h.ns_u, bas_u, knots_v_dev, q, idx_v, h.ns_v, bas_v, st);
   if (e == cudaSuccess) e = launch_span_matrices(d, bas_u, bas_v, matrix_n_dev, nullptr, st);
   return e == cudaSuccess ? NURBS_OK : cuda_fail(e, "matrix-form conversion");
 }

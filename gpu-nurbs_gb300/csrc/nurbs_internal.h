@@ -14,6 +14,10 @@ __host__ __device__ inline int span_coefs32(int p, int q) {
   const int k = (p + 1) * (q + 1);
   return k + (k & 1);
 }
+// Spans converted by one CTA of the span-matrix kernel: a thread per (span, column, component).
+constexpr int kSpanGroupThreads = 128;
+__host__ __device__ inline int span_group(int q) { return kSpanGroupThreads / (4 * (q + 1)); }
+inline int64_t span_blocks(int q, int64_t nspans) { return (nspans + span_group(q) - 1) / span_group(q); }
 constexpr int kGap = 8;           // GapPerEdge (src/kernel/kernel.cuh:17)
 constexpr int kPts = kGap + 1;    // PointsPerEdge
 constexpr int kConeStride = 20;   // floats per normal-cone record
@@ -94,8 +98,9 @@ int cuda_fail(cudaError_t e, const char* what);
 
 // ---- launchers (each returns a cudaError_t from the launch) ----
 // stage a
-cudaError_t launch_basis(const double* knots, int degree, const int* knot_idx, int nspans,
-                         double* basis_out, cudaStream_t st);
+cudaError_t launch_basis_pair(const double* knots_u, int p, const int* idx_u, int ns_u, double* basis_u,
+                              const double* knots_v, int q, const int* idx_v, int ns_v, double* basis_v,
+                              cudaStream_t st);
 cudaError_t launch_span_matrices(const SurfDev& s, const double* basis_u, const double* basis_v,
                                  double* m64, float* m32, cudaStream_t st);
 cudaError_t launch_export_ref_layout(const SurfDev& s, double* matrix_n, cudaStream_t st);
@@ -112,18 +117,19 @@ cudaError_t launch_evaluate_random(const double* uv, double* xyz, int64_t n, con
                                    int q, int nu, int nv, const double* knots_u, const double* knots_v,
                                    cudaStream_t st);
 // stage c
-cudaError_t launch_tree(const SurfDev& s, cudaStream_t st);
+// tree, normal cones, bound boxes, lattice points and quadtree boxes, after the span tables
+cudaError_t launch_nodes(const SurfDev& s, cudaStream_t st);
 cudaError_t launch_candidates(const SurfDev& s, const double* P, int64_t n, int* list, int* counts,
                               cudaStream_t st);
 // batched (pool) variants: surfaces are read from a device table of SurfDev records
-struct BasisJob {        // one (surface, direction): its spans' columns are items [item0, item0 + ns*(d+1))
+struct BasisJob {        // one (surface, direction): its spans are items [item0, item0 + nspans)
   const double* knots;
   const int* knot_idx;
   double* out;
   int degree, nspans;
   int64_t item0;
 };
-struct SpanJob {         // one surface: its spans x 4 components are items [item0, item0 + 4*ns_u*ns_v)
+struct SpanJob {         // one surface: its groups of spans are items [item0, item0 + span_blocks(q, ns_u*ns_v))
   int surf;
   int64_t item0;
 };
@@ -132,10 +138,10 @@ struct InvTile {         // a range of queries of one surface
   int count;
   int64_t begin;
 };
-cudaError_t launch_basis_batched(const BasisJob* jobs, int njobs, int64_t nitems, cudaStream_t st);
-cudaError_t launch_span_matrices_batched(const SurfDev* table, const SpanJob* jobs, int njobs, int64_t nitems,
+cudaError_t launch_basis_batched(const BasisJob* jobs, int njobs, int64_t nspans, cudaStream_t st);
+cudaError_t launch_span_matrices_batched(const SurfDev* table, const SpanJob* jobs, int njobs, int64_t nblocks,
                                          cudaStream_t st);
-cudaError_t launch_tree_batched(const SurfDev* table, const int* ids, int count, cudaStream_t st);
+cudaError_t launch_nodes_batched(const SurfDev* table, const int* ids, int count, cudaStream_t st);
 cudaError_t launch_eval_pool(const SurfDev* table, const InvTile* tiles, int ntiles, const double* uv, int64_t n,
                              unsigned mask, double* out, cudaStream_t st);
 cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int ntiles, int* counter,
@@ -149,14 +155,10 @@ cudaError_t launch_invert(const SurfDev& s, const double* P, int64_t n, double* 
 cudaError_t launch_pcurve_passes(const SurfDev& s, const double* C, int64_t n, const double* uv0, const int* st0,
                                  const double* res0, double* uv, int* st, double* res, int* flags,
                                  cudaStream_t stream);
-// normal cones, bound boxes and lattice points of the built nodes (after the tree and the span tables)
-cudaError_t launch_cones(const SurfDev& s, cudaStream_t st);
 // the projection: closest point over the closed domain (k_project.cu)
 cudaError_t launch_project(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
                            double* residual, int precision, unsigned* counter, cudaStream_t st);
-// adaptive quadtree inversion (k_quadtree.cu); its top levels' control-point boxes (qtbox), written
-// with the tree
-cudaError_t launch_quadtree_boxes(const SurfDev& s, cudaStream_t st);
+// adaptive quadtree inversion (k_quadtree.cu)
 cudaError_t launch_invert_quadtree(const SurfDev& s, const double* P, int64_t n, double max_edge, double* uv,
                                    int* status, double* residual, int precision, unsigned* counter, cudaStream_t st);
 // S, Su, Sv at the built nodes' uv-centres (cd32/cd64), after the tree is built

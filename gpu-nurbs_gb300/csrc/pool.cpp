@@ -384,11 +384,11 @@ int nurbs_pool_add(nurbs_pool_t P, int count, const nurbs_surface_desc* descs, v
     fill_surface(S[k], img.data() + o, P->base + in_off + o, P->base + out_off[k], recs[k]);
     const SurfDev& d = recs[k];
     bjobs.push_back(BasisJob{d.knots_u, d.knot_u, d.basis_u, d.p, d.ns_u, bitems});
-    bitems += (int64_t)d.ns_u * (d.p + 1);
+    bitems += d.ns_u;
     bjobs.push_back(BasisJob{d.knots_v, d.knot_v, d.basis_v, d.q, d.ns_v, bitems});
-    bitems += (int64_t)d.ns_v * (d.q + 1);
+    bitems += d.ns_v;
     sjobs.push_back(SpanJob{ids[k], sitems});
-    sitems += (int64_t)d.ns_u * d.ns_v * 4;
+    sitems += span_blocks(d.q, (int64_t)d.ns_u * d.ns_v);
     o += S[k].in_bytes;
   }
   std::vector<char> scr(scratch_bytes, 0);
@@ -403,7 +403,7 @@ int nurbs_pool_add(nurbs_pool_t P, int count, const nurbs_surface_desc* descs, v
   if (e == cudaSuccess) e = launch_basis_batched((const BasisJob*)sdev, (int)bjobs.size(), bitems, st);
   if (e == cudaSuccess)
     e = launch_span_matrices_batched(P->d_table, (const SpanJob*)(sdev + jb), (int)sjobs.size(), sitems, st);
-  if (e == cudaSuccess) e = launch_tree_batched(P->d_table, (const int*)(sdev + jb + js), count, st);
+  if (e == cudaSuccess) e = launch_nodes_batched(P->d_table, (const int*)(sdev + jb + js), count, st);
   if (e == cudaSuccess) e = launch_centre_ders_batched(P->d_table, (const int*)(sdev + jb + js), count, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // host images must outlive the copies
   // 4. publication (locked)
