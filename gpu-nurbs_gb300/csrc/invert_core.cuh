@@ -40,6 +40,9 @@ constexpr int kSmemSpans = 256;         // breakpoint tables staged in shared me
 // Which lane runs which seed, and when, does not change any seed's arithmetic, and the
 // records are independent of arrival order, so results are the same for every value.
 constexpr int kStartBatch = 8;
+// The FP64 schedule's (50,021 queries of the 64x64 surface: 1 / 3 / 6 / 10 take 7.52 / 7.38 / 7.47 /
+// 7.73 ms).
+constexpr int kStartBatch64 = 3;
 
 // Arithmetic below writes every product that feeds a sum as an explicit FMA (the translation
 // units are compiled with --fmad=false), so a seed's trajectory is the same bit for bit in
@@ -70,7 +73,7 @@ __device__ __forceinline__ int solve_step(const v3<T>& r, const v3<T>& Su, const
   int kind = kStepGN;
   if (newton) {
     const T n00 = h00 + dot3c(r, Suu), n01 = h01 + dot3c(r, Suv), n11 = h11 + dot3c(r, Svv);
-    if (n00 > T(0) && det2(n00, n01, n11) > T(0)) {
+    if (fast::is_positive(n00) && fast::is_positive(det2(n00, n01, n11))) {
       h00 = n00;
       h01 = n01;
       h11 = n11;
@@ -78,7 +81,7 @@ __device__ __forceinline__ int solve_step(const v3<T>& r, const v3<T>& Su, const
     }
   }
   const T det = det2(h00, h01, h11);
-  if (!(det > T(0))) return kSingular;
+  if (!fast::is_positive(det)) return kSingular;
   const T inv = fast::rcp<FAST>(det);
   du = fast::mad(h11, g0, -(h01 * g1)) * inv;
   dv = fast::mad(h00, g1, -(h01 * g0)) * inv;
@@ -135,22 +138,39 @@ __device__ __forceinline__ int iterate32(const Ctx& c, float px, float py, float
   return kContinue;
 }
 
-// One FP64 iteration of a seed (FP64 mode).
+// One FP64 iteration of a seed (FP64 mode).  dist2, when the seed converges: |S - P|^2 at the new
+// (u, v) from this step's S, Su, Sv: S(u - du, v - dv) = S - Su du - Sv dv + O(|S''| 1e-20), below
+// the rounding of S itself (another evaluation for the few lanes whose seeds just ended would cost
+// the warp as much as one for all lanes).
 template <int P, int Q>
-__device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, double pz, Seed<double>& st) {
+__device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, double pz, Seed<double>& st,
+                                         double& dist2) {
   fast::SDer<double> d = fast::eval_at<double, P, Q, 2>(c.L64, c.m64, c.p, c.q, st.u, st.v, st.hu, st.hv);
   v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   double du, dv;
   if (!solve_step<double, double, false>(r, d.Su, d.Sv, d.Suu, d.Suv, d.Svv, st.newton, du, dv)) return kFailed;
-  if (!(isfinite(du) && isfinite(dv))) return kFailed;
+  if (!(fast::is_finite(du) && fast::is_finite(dv))) return kFailed;
   st.u -= du;
   st.v -= dv;
-  double step = fmax(fabs(du), fabs(dv));
-  if ((st.newton && step <= kTolNewton64) || step <= kTolAny64) return kConverged;
+  const double step = fast::max_abs(du, dv);
+  if ((st.newton && fast::le_nonneg(step, kTolNewton64)) || fast::le_nonneg(step, kTolAny64)) {
+    const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
+                           fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
+                           fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
+    dist2 = dot3(r2, r2);
+    return kConverged;
+  }
   st.prev = step;
-  st.newton = step < kNewtonSwitch;
+  st.newton = fast::lt_nonneg(step, kNewtonSwitch);
   if (++st.it >= kMaxIter64) return kFailed;
   return kContinue;
+}
+
+// An FP64 seed's end counts when it lies in the domain at a finite distance.
+__device__ __forceinline__ bool in_domain64(const Ctx& c, double u, double v, double dist2) {
+  const long long ku = fast::order_key(u), kv = fast::order_key(v);
+  return ku >= fast::order_key(c.dom_u0) && ku <= fast::order_key(c.dom_u1) && kv >= fast::order_key(c.dom_v0) &&
+         kv <= fast::order_key(c.dom_v1) && fast::is_finite(dist2);
 }
 
 // The first iteration of a seed from its node centre's precomputed S, Su, Sv (cd = 9 values,
@@ -165,11 +185,15 @@ __device__ __forceinline__ void first_step(const T* __restrict__ cd, T px, T py,
   const v3<T> r = {S.x - px, S.y - py, S.z - pz};
   T du, dv;
   if (solve_step<T, T, sizeof(T) == 4>(r, Su, Sv, Su, Su, Su, false, du, dv) == kSingular) return;
-  if (!(isfinite(du) && isfinite(dv))) return;
   const T u = st.u - du, v = st.v - dv;
   T step;
-  if constexpr (sizeof(T) == 4) step = fmaxf(fabsf(du), fabsf(dv));
-  else step = fmax(fabs(du), fabs(dv));
+  if constexpr (sizeof(T) == 4) {
+    if (!(isfinite(du) && isfinite(dv))) return;
+    step = fmaxf(fabsf(du), fabsf(dv));
+  } else {
+    if (!(fast::is_finite(du) && fast::is_finite(dv))) return;
+    step = fast::max_abs(du, dv);
+  }
   if constexpr (sizeof(T) == 4) {
     const float smag = fmaxf(fmaxf(fabsf(S.x), fabsf(S.y)), fmaxf(fabsf(S.z), 1.0f));
     const v3<float> dS = {fast::mad(Sv.x, dv, Su.x * du), fast::mad(Sv.y, dv, Su.y * du),
@@ -178,23 +202,14 @@ __device__ __forceinline__ void first_step(const T* __restrict__ cd, T px, T py,
     if (step <= kTol32 || dot3(dS, dS) <= fl * fl) return;  // converged at once: left to iterate32
     if (!(u >= far[0] && u <= far[1] && v >= far[2] && v <= far[3])) return;
   } else {
-    if (step <= kTolAny64) return;
+    if (fast::le_nonneg(step, kTolAny64)) return;
   }
   st.u = u;
   st.v = v;
   st.prev = step;
-  st.newton = step < (T)kNewtonSwitch;
+  if constexpr (sizeof(T) == 4) st.newton = step < (T)kNewtonSwitch;
+  else st.newton = fast::lt_nonneg(step, kNewtonSwitch);
   st.it = 1;
-}
-
-// FP64 residual at (u,v), with the domain test.
-template <int P, int Q>
-__device__ __forceinline__ bool finish64(const Ctx& c, double px, double py, double pz, double u, double v,
-                                         int hu, int hv, double& res) {
-  fast::SDer<double> d = fast::eval_at<double, P, Q, 0>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
-  v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
-  res = sqrt(dot3(r, r));
-  return (u >= c.dom_u0 && u <= c.dom_u1 && v >= c.dom_v0 && v <= c.dom_v1) && isfinite(res);
 }
 
 // MIXED: the final FP64 Newton steps from an FP32 minimum, then the residual.  The first
@@ -225,17 +240,18 @@ __device__ bool final64(const Ctx& c, double px, double py, double pz, double& u
       kind = solve_step<double, double, false>(r, d.Su, d.Sv, d.Suu, d.Suv, d.Svv, true, du, dv);
     }
     if (kind == kSingular) return false;
-    if (!(isfinite(du) && isfinite(dv))) return false;
+    if (!(fast::is_finite(du) && fast::is_finite(dv))) return false;
     u -= du;
     v -= dv;
-    if (fmax(fabs(du), fabs(dv)) <= kTolNewton64) {
+    if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
       // Residual at the returned point from this step's FP64 S, Su, Sv: S(u - du, v - dv) =
       // S - Su du - Sv dv + O(|S''| 1e-20), below the rounding of S itself.
       const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
                              fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
                              fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-      res = sqrt(dot3(r2, r2));
-      return (u >= c.dom_u0 && u <= c.dom_u1 && v >= c.dom_v0 && v <= c.dom_v1) && isfinite(res);
+      const double dist2 = dot3(r2, r2);
+      res = sqrt(dist2);
+      return in_domain64(c, u, v, dist2);
     }
   }
   return false;
@@ -271,9 +287,12 @@ struct Rec32 {  // per-query FP32 record: best and best distinct runner-up (squa
 // the order in which its members arrive, so per-query records are schedule independent.
 template <typename T>
 __device__ __forceinline__ bool before(T d, T u, T v, T d0, T u0, T v0) {
-  return d < d0 || (d == d0 && (u < u0 || (u == u0 && v < v0)));
+  const auto kd = fast::order_key(d), kd0 = fast::order_key(d0);
+  if (kd != kd0) return kd < kd0;
+  const auto ku = fast::order_key(u), ku0 = fast::order_key(u0);
+  return ku < ku0 || (ku == ku0 && fast::order_key(v) < fast::order_key(v0));
 }
-struct Rec64 {  // per-query FP64 record: distinct minima and their grid cells
+struct Rec64 {  // per-query FP64 record: distinct minima (r: squared distances) and their grid cells
   double u[kSols], v[kSols], r[kSols];
   int cu[kSols], cv[kSols];
   int n;
@@ -704,33 +723,41 @@ __device__ __forceinline__ void invert_chunk(Staged<KS, MODE>& sm, WarpWork<MODE
         first_step<double>(sm.cd64 + 9 * node, tx, ty, tz, sm.far32, sd);
       };
       if (active) start();
-      while (__any_sync(FULL, active)) {
-        int res = kContinue;
-        double rr = 0;
-        bool keep = false;
+      // lanes whose seed has ended wait until kStartBatch64 are free: their results are merged and
+      // their next seeds started together (the first step is as much FP64 work for one lane as for
+      // all)
+      bool waiting = false, keep = false;
+      double rr = 0;
+      while (__any_sync(FULL, active || waiting)) {
         if (active) {
-          res = iterate64<P, Q>(cx, tx, ty, tz, sd);
+          const int res = iterate64<P, Q>(cx, tx, ty, tz, sd, rr);
           if constexpr (COUNT) ++n_iter;
-          if (res == kConverged) keep = finish64<P, Q>(cx, tx, ty, tz, sd.u, sd.v, sd.hu, sd.hv, rr);
+          if (res != kContinue) {
+            keep = res == kConverged && in_domain64(cx, sd.u, sd.v, rr);
+            active = false;
+            waiting = true;
+          }
         }
-        const bool done = active && res != kContinue;
-        __syncwarp();
-        int cu = 0, cv = 0;
-        if (done && keep) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
-        unsigned fm = __ballot_sync(FULL, done && keep);
-        while (fm) {
-          int j = __ffs(fm) - 1;
-          if (lane == j) merge64(ww.rec[ql], cu, cv, sd.u, sd.v, rr);
-          __syncwarp();
-          fm &= fm - 1;
+        const unsigned wm = __ballot_sync(FULL, waiting);
+        if (wm && (__popc(wm) >= kStartBatch64 || !__any_sync(FULL, active))) {
+          int cu = 0, cv = 0;
+          if (waiting && keep) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
+          unsigned fm = __ballot_sync(FULL, waiting && keep);
+          while (fm) {
+            int j = __ffs(fm) - 1;
+            if (lane == j) merge64(ww.rec[ql], cu, cv, sd.u, sd.v, rr);
+            __syncwarp();
+            fm &= fm - 1;
+          }
+          if (waiting) {
+            task = next + __popc(wm & lt_mask);
+            active = task < total;
+            waiting = false;
+            keep = false;
+            if (active) start();
+          }
+          next += __popc(wm);
         }
-        unsigned dm = __ballot_sync(FULL, done);
-        if (done) {
-          task = next + __popc(dm & lt_mask);
-          active = task < total;
-          if (active) start();
-        }
-        next += __popc(dm);
       }
     }
     __syncwarp();
@@ -788,7 +815,9 @@ __device__ __forceinline__ void invert_chunk(Staged<KS, MODE>& sm, WarpWork<MODE
       status = ns == 0 ? 3 : finish_status(us, vs, rs, ns, kDistinct, kDistinct, ou, ov, orr);
     } else {
       const Rec64& R = ww.rec[lane];
-      status = R.n == 0 ? 3 : finish_status(R.u, R.v, R.r, R.n, 2.0 / sm.cell64.iu, 2.0 / sm.cell64.iv, ou, ov, orr);
+      double rs[kSols];
+      for (int k = 0; k < kSols; ++k) rs[k] = k < R.n ? sqrt(R.r[k]) : 0.0;
+      status = R.n == 0 ? 3 : finish_status(R.u, R.v, rs, R.n, 2.0 / sm.cell64.iu, 2.0 / sm.cell64.iv, ou, ov, orr);
     }
     if (valid) {
       uv_out[2 * q] = ou;

@@ -63,11 +63,13 @@ __device__ bool continue_from(const Ctx& cx, double px, double py, double pz, do
   sd.hv = 0;
   sd.newton = true;
   int r = kContinue;
-  while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd);
+  double dist2 = 0;
+  while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd, dist2);
   if (r != kConverged) return false;
   u = sd.u;
   v = sd.v;
-  return finish64<P, Q>(cx, px, py, pz, u, v, sd.hu, sd.hv, res);
+  res = sqrt(dist2);
+  return in_domain64(cx, u, v, dist2);
 }
 
 template <int P, int Q>

@@ -129,6 +129,16 @@ __device__ __forceinline__ int project_iterate32(const Ctx& c, const float dom[4
   return kContinue;
 }
 
+// FP64 residual at (u,v), with the domain test.
+template <int P, int Q>
+__device__ __forceinline__ bool finish64(const Ctx& c, double px, double py, double pz, double u, double v,
+                                         int hu, int hv, double& res) {
+  fast::SDer<double> d = fast::eval_at<double, P, Q, 0>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
+  v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
+  res = sqrt(dot3(r, r));
+  return (u >= c.dom_u0 && u <= c.dom_u1 && v >= c.dom_v0 && v <= c.dom_v1) && isfinite(res);
+}
+
 // One projected Newton iteration with its line search (see above).
 template <int P, int Q>
 __device__ __forceinline__ int project_iterate(const Ctx& c, double px, double py, double pz, PSeed& sd) {

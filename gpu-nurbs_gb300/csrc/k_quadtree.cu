@@ -184,10 +184,13 @@ __device__ bool node_trajectory(const SurfDev& s, const Ctx& cx, double px, doub
     sd.hv = 0;
     sd.newton = false;
     int r = kContinue;
-    while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd);
+    double dist2 = 0;
+    while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd, dist2);
     u = sd.u;
     v = sd.v;
-    return r == kConverged && finish64<P, Q>(cx, px, py, pz, u, v, sd.hu, sd.hv, rr) && rr < max_edge;
+    if (r != kConverged || !in_domain64(cx, u, v, dist2)) return false;
+    rr = sqrt(dist2);
+    return rr < max_edge;
   }
 }
 
