@@ -133,7 +133,7 @@ struct nurbs_surface_s {
   double* basis_v = nullptr;
   int device = 0;
   bool tree_built = false;
-  unsigned* counters = nullptr;  // kCounterRing device words
+  unsigned long long* counters = nullptr;  // kCounterRing device words
   cudaEvent_t done[kCounterRing] = {};
   unsigned next_slot = 0;
   std::mutex mu;
@@ -163,7 +163,7 @@ static cudaError_t invert_on(nurbs_surface_s* s, const double* P, int64_t n, dou
       if (e != cudaSuccess) return e;
     }
   }
-  e = cudaMemsetAsync(s->counters + slot, 0, sizeof(unsigned), st);
+  e = cudaMemsetAsync(s->counters + slot, 0, sizeof(unsigned long long), st);
   if (e == cudaSuccess) {
     if (op == QueryOp::kQuadtree)
       e = launch_invert_quadtree(s->dev, P, n, max_edge, uv, status, res, precision, s->counters + slot, st);
@@ -256,6 +256,8 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
   if (e == cudaSuccess) e = launch_span_matrices(d, s->basis_u, s->basis_v, (double*)d.m64, (float*)d.m32, st);
   if (e == cudaSuccess) e = launch_nodes(d, st);
   if (e == cudaSuccess) e = launch_centre_ders(d, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&d.seeds, d.cd32 + 9 * kTreeNodes, sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // img must outlive the copy
   if (e != cudaSuccess) {
     cudaFree(s->arena);
@@ -263,7 +265,7 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
     return cuda_fail(e, "matrix-form conversion");
   }
   s->tree_built = true;
-  e = cudaMalloc((void**)&s->counters, sizeof(unsigned) * kCounterRing);
+  e = cudaMalloc((void**)&s->counters, sizeof(unsigned long long) * kCounterRing);
   if (e != cudaSuccess) {
     cudaFree(s->arena);
     delete s;
@@ -403,6 +405,8 @@ int nurbs_build_tree(nurbs_surface_t s, int levels, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   CUDA_TRY(launch_nodes(s->dev, st), "tree launch");
   CUDA_TRY(launch_centre_ders(s->dev, st), "seed-centre derivatives");
+  CUDA_TRY(cudaMemcpyAsync(&s->dev.seeds, s->dev.cd32 + 9 * kTreeNodes, sizeof(float), cudaMemcpyDeviceToHost, st),
+           "average candidates");
   CUDA_TRY(cudaStreamSynchronize(st), "tree sync");
   s->tree_built = true;
   return NURBS_OK;
@@ -519,7 +523,7 @@ int nurbs_invert_count(nurbs_surface_t s, const double* P_dev, int64_t n, int pr
                total = oR + align256((size_t)n * 8);
   char* buf = nullptr;
   CUDA_TRY(tmp_alloc((void**)&buf, total, st), "device buffers");
-  unsigned* counter = (unsigned*)buf;
+  unsigned long long* counter = (unsigned long long*)buf;
   unsigned long long* counts = (unsigned long long*)(buf + 64);
   cudaError_t e = cudaMemsetAsync(buf, 0, 256, st);
   if (e == cudaSuccess)

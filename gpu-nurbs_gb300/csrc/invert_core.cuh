@@ -16,7 +16,6 @@ constexpr int kModeMixed = 1;
 
 constexpr int kWarps = 4;          // warps per CTA
 constexpr int kThreads = 32 * kWarps;
-constexpr int kMinBlocksMixed = 6;  // CTAs per SM the mixed kernels are register-budgeted for (80 registers)
 constexpr int kMaxIter32 = 40;     // FP32 iterations per seed (the FP64 cap: the oracle's too)
 constexpr int kMaxIter64 = 40;     // FP64-mode iterations per seed
 constexpr int kMaxFinal64 = 24;    // MIXED: FP64 steps (2 normally)
@@ -35,7 +34,7 @@ constexpr float kDistinct32 = 1e-4f;    // FP32 minima: the same
 constexpr int kSols = 4;                // FP64 mode: distinct minima kept per query
 constexpr int kSmemSpans = 256;         // breakpoint tables staged in shared memory up to this
 // MIXED: lanes whose seed has ended wait until this many are free (or no lane still iterates)
-// and then start their next seeds together, so that the divergent start (task decode, the first
+// and then merge their results and start their next seeds together, so that the divergent start (task decode, the first
 // step from the node centre) runs once for several lanes instead of every iteration for ~3.
 // Which lane runs which seed, and when, does not change any seed's arithmetic, and the
 // records are independent of arrival order, so results are the same for every value.
@@ -43,6 +42,16 @@ constexpr int kStartBatch = 8;
 // The FP64 schedule's (50,021 queries of the 64x64 surface: 1 / 3 / 6 / 10 take 7.52 / 7.38 / 7.47 /
 // 7.73 ms).
 constexpr int kStartBatch64 = 3;
+// Slots free or finished before the task list is refilled while seeds still run.  A refill of the
+// mixed schedule passes its finished queries through the final FP64 steps, as long for one lane as
+// for all: 24 / 28 / 29 slots take 1.52 / 1.39 / 1.42 ms on the 8x8 surface (2^20 queries), the same on
+// the 64x64 one.  The FP64 schedule has no such pass.
+constexpr int kRefillMixed = 28;
+constexpr int kRefill64 = 8;
+// Seeds a warp's least portion holds (least_grab).  Mixed, 32 / 64: 64x64 surface, 6,000 queries 230 /
+// 210 us; 8x8 surface, 60,000 queries 145 / 126 us; FP64 64 / 128: 50,021 queries 6.73 / 6.67 ms.
+constexpr float kGrabSeedsMixed = 64, kGrabSeeds64 = 128;
+constexpr int kSchedulers = 4 * 152;  // of the GB300: four per SM, an FP64 pipe each
 
 // Arithmetic below writes every product that feeds a sum as an explicit FMA (the translation
 // units are compiled with --fmad=false), so a seed's trajectory is the same bit for bit in
@@ -98,6 +107,21 @@ struct Ctx {
   double dom_u0, dom_u1, dom_v0, dom_v1;
 };
 
+// The FP32 evaluation of S..Svv that the explorations iterate with, from a context's tables
+// (GlobalEval: breakpoints by bisection from the last span) or from a staged surface (StagedEval).
+template <int P, int Q>
+struct GlobalEval {
+  const Ctx& c;
+  __device__ __forceinline__ void spans(float u, float v, int& hu, int& hv) const {
+    hu = fast::find_seg_hint(c.L32.bu, c.L32.ns_u, u, hu);
+    hv = fast::find_seg_hint(c.L32.bv, c.L32.ns_v, v, hv);
+  }
+  template <int ORDER>
+  __device__ __forceinline__ fast::SDer<float> at(float u, float v, int& hu, int& hv) const {
+    return fast::eval_at<float, P, Q, ORDER, true>(c.L32, c.m32, c.p, c.q, u, v, hu, hv);
+  }
+};
+
 // Per-seed iteration state (hu/hv: span hints for the warm-started span search).
 template <typename T>
 struct Seed {
@@ -114,9 +138,9 @@ enum StepResult { kContinue = 0, kConverged = 1, kFailed = 2 };
 // positive definite the iterate is near a saddle of the distance, from which the GN steps creep
 // away slowly: steps that do not shrink there are no sign of convergence.  dist2 = |S - P|^2
 // before the step.
-template <int P, int Q>
-__device__ __forceinline__ int iterate32(const Ctx& c, float px, float py, float pz, Seed<float>& st, float& dist2) {
-  fast::SDer<float> d = fast::eval_at<float, P, Q, 2, true>(c.L32, c.m32, c.p, c.q, st.u, st.v, st.hu, st.hv);
+template <class Eval>
+__device__ __forceinline__ int iterate32(const Eval& ev, float px, float py, float pz, Seed<float>& st, float& dist2) {
+  fast::SDer<float> d = ev.template at<2>(st.u, st.v, st.hu, st.hv);
   v3<float> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   float du, dv;
   const int kind = solve_step<float, float, true>(r, d.Su, d.Sv, d.Suu, d.Suv, d.Svv, st.newton, du, dv);
@@ -217,44 +241,66 @@ __device__ __forceinline__ void first_step(const T* __restrict__ cd, T px, T py,
 // sets the rate of convergence, and two steps normally reach the tolerance); later steps take
 // it in FP64, which converges where the minimum is nearly degenerate (a flat valley, where the
 // FP32 term's error is comparable to the Hessian's smallest eigenvalue).
-template <int P, int Q>
-__device__ bool final64(const Ctx& c, double px, double py, double pz, double& u, double& v, double& res) {
+struct Final {
+  double u, v;
+  int it, hu, hv, hu32, hv32;
+};
+template <class Eval>
+__device__ __forceinline__ void final_start(const Eval& ev, double u, double v, Final& f) {
+  f.u = u;
+  f.v = v;
+  f.it = 0;
   // span hints from the FP32 tables (shared memory when staged): the FP64 search then only
   // confirms them with two reads instead of bisecting the FP64 tables in global memory
-  int hu = fast::find_seg_hint(c.L32.bu, c.L32.ns_u, (float)u, 0);
-  int hv = fast::find_seg_hint(c.L32.bv, c.L32.ns_v, (float)v, 0);
-  int hu32 = hu, hv32 = hv;
-  for (int it = 0; it < kMaxFinal64; ++it) {
-    fast::SDer<double> d;
-    double du, dv;
-    int kind;
-    v3<double> r;
-    if (it < kFinal32Curv) {
-      d = fast::eval_at<double, P, Q, 1>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
-      fast::SDer<float> e = fast::eval_at<float, P, Q, 2, true>(c.L32, c.m32, c.p, c.q, (float)u, (float)v, hu32, hv32);
-      r = {d.S.x - px, d.S.y - py, d.S.z - pz};
-      kind = solve_step<double, float, false>(r, d.Su, d.Sv, e.Suu, e.Suv, e.Svv, true, du, dv);
-    } else {
-      d = fast::eval_at<double, P, Q, 2>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
-      r = {d.S.x - px, d.S.y - py, d.S.z - pz};
-      kind = solve_step<double, double, false>(r, d.Su, d.Sv, d.Suu, d.Suv, d.Svv, true, du, dv);
-    }
-    if (kind == kSingular) return false;
-    if (!(fast::is_finite(du) && fast::is_finite(dv))) return false;
-    u -= du;
-    v -= dv;
-    if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
-      // Residual at the returned point from this step's FP64 S, Su, Sv: S(u - du, v - dv) =
-      // S - Su du - Sv dv + O(|S''| 1e-20), below the rounding of S itself.
-      const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
-                             fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
-                             fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-      const double dist2 = dot3(r2, r2);
-      res = sqrt(dist2);
-      return in_domain64(c, u, v, dist2);
-    }
+  f.hu = f.hv = 0;
+  ev.spans((float)u, (float)v, f.hu, f.hv);
+  f.hu32 = f.hu;
+  f.hv32 = f.hv;
+}
+// One step: kConverged (in the domain, res the residual), kFailed or kContinue.
+template <int P, int Q, class Eval>
+__device__ __forceinline__ int final_step(const Ctx& c, const Eval& ev, double px, double py, double pz, Final& f,
+                                          double& res) {
+  fast::SDer<double> d;
+  double du, dv;
+  int kind;
+  v3<double> r;
+  if (f.it < kFinal32Curv) {
+    d = fast::eval_at<double, P, Q, 1>(c.L64, c.m64, c.p, c.q, f.u, f.v, f.hu, f.hv);
+    fast::SDer<float> e = ev.template at<2>((float)f.u, (float)f.v, f.hu32, f.hv32);
+    r = {d.S.x - px, d.S.y - py, d.S.z - pz};
+    kind = solve_step<double, float, false>(r, d.Su, d.Sv, e.Suu, e.Suv, e.Svv, true, du, dv);
+  } else {
+    d = fast::eval_at<double, P, Q, 2>(c.L64, c.m64, c.p, c.q, f.u, f.v, f.hu, f.hv);
+    r = {d.S.x - px, d.S.y - py, d.S.z - pz};
+    kind = solve_step<double, double, false>(r, d.Su, d.Sv, d.Suu, d.Suv, d.Svv, true, du, dv);
   }
-  return false;
+  if (kind == kSingular) return kFailed;
+  if (!(fast::is_finite(du) && fast::is_finite(dv))) return kFailed;
+  f.u -= du;
+  f.v -= dv;
+  if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
+    // Residual at the returned point from this step's FP64 S, Su, Sv: S(u - du, v - dv) =
+    // S - Su du - Sv dv + O(|S''| 1e-20), below the rounding of S itself.
+    const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
+                           fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
+                           fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
+    const double dist2 = dot3(r2, r2);
+    res = sqrt(dist2);
+    return in_domain64(c, f.u, f.v, dist2) ? kConverged : kFailed;
+  }
+  return ++f.it < kMaxFinal64 ? kContinue : kFailed;
+}
+template <int P, int Q>
+__device__ bool final64(const Ctx& c, double px, double py, double pz, double& u, double& v, double& res) {
+  Final f;
+  const GlobalEval<P, Q> ev{c};
+  final_start(ev, u, v, f);
+  int r = kContinue;
+  while (r == kContinue) r = final_step<P, Q>(c, ev, px, py, pz, f, res);
+  u = f.u;
+  v = f.v;
+  return r == kConverged;
 }
 
 // Position of the k-th (0-based) set bit of m, which has more than k set bits: a fixed
@@ -389,63 +435,172 @@ struct Staged {
   Cells<float> cell32;
   Cells<double> cell64;
   int nb;
-  float sb32[2][KS + 1], si32[2][KS];
+  Ctx ctx;      // the surface's context: one copy for all threads, its fields read where they are used
+  bool fits;    // breakpoint tables staged (at most KS spans per direction)
+  // FP32 breakpoints and inverse span lengths, and a lookup grid over the domain: KS equal buckets,
+  // each with the span of its left end (or one before)
+  float2 seg[2][KS + 1];
+  float g0[2], gs[2];  // bucket of x: (x - g0) * gs
+  unsigned char grid[2][KS];
   double sb64[2][KS64 + 1], si64[2][KS64];
+
+  // The span of x, as find_seg_hint's: two or three dependent shared-memory reads instead of a
+  // bisection's 6 to 8 (which the whole warp runs as soon as one lane has left its last span; the
+  // bisections took a quarter of an iteration of the exploration).
+  __device__ __forceinline__ int span(int dir, int ns, float x) const {
+    const int i = min(max((int)((x - g0[dir]) * gs[dir]), 0), KS - 1);
+    int k = grid[dir][i];
+    for (int n = 0; k < ns - 1 && x >= seg[dir][k + 1].x; ++n) {
+      ++k;
+      if (n == 3) {  // clustered knots
+        for (int step = 1 << (31 - __clz(ns)); step > 0; step >>= 1)
+          if (k + step < ns && seg[dir][k + step].x <= x) k += step;
+        break;
+      }
+    }
+    return k;
+  }
 };
 
-// Per-warp bookkeeping of the task scheduler: candidate masks, task-order tables, per-query
-// records and query coordinates of the warp's (up to) 32 queries.
+template <int P, int Q, int KS, int MODE>
+struct StagedEval {
+  const Staged<KS, MODE>& sm;
+  __device__ __forceinline__ void spans(float u, float v, int& hu, int& hv) const {
+    if (sm.fits) {
+      hu = sm.span(0, sm.ctx.L32.ns_u, u);
+      hv = sm.span(1, sm.ctx.L32.ns_v, v);
+    } else {
+      GlobalEval<P, Q>{sm.ctx}.spans(u, v, hu, hv);
+    }
+  }
+  template <int ORDER>
+  __device__ __forceinline__ fast::SDer<float> at(float u, float v, int& hu, int& hv) const {
+    const fast::Locator<float>& L = sm.ctx.L32;
+    float bu, bv, iu, iv;
+    spans(u, v, hu, hv);
+    if (sm.fits) {
+      const float2 a = sm.seg[0][hu], b = sm.seg[1][hv];
+      bu = a.x;
+      iu = a.y;
+      bv = b.x;
+      iv = b.y;
+    } else {
+      bu = L.bu[hu];
+      iu = L.iu[hu];
+      bv = L.bv[hv];
+      iv = L.iv[hv];
+    }
+    const float lu = (u - bu) * iu, lv = (v - bv) * iv;
+    return fast::eval_span<float, P, Q, ORDER, true>(sm.ctx.m32, sm.ctx.p, sm.ctx.q, L.ns_v, hu, hv, lu, lv, L.ru * iu,
+                                                     L.rv * iv);
+  }
+};
+
+// Per-warp bookkeeping of the task scheduler: the warp's 32 query slots.
 template <int MODE>
 struct WarpWork {
-  unsigned long long smask0[32];
-  unsigned char smask1[32];
-  // round-major task order and the queries' FP64 coordinates: FP64 schedule only
-  unsigned srmask[MODE == kModeMixed ? 1 : kTreeNodes];
-  int srpref[MODE == kModeMixed ? 1 : kTreeNodes + 1];
-  int slpref[32];
+  long long sq[32];              // query index of the slot
+  unsigned long long smask0[32]; // candidate nodes 0..63 of the slots in the current task list
+  int slpref[32];                // exclusive prefix of the slots' task counts
+  int sleft[32];                 // seeds of the slot's query that have not ended
   typename std::conditional<MODE == kModeMixed, Rec32, Rec64>::type rec[32];
-  float sp32[32][3];
+  float sp32[MODE == kModeMixed ? 32 : 1][3];
   double sp64[MODE == kModeMixed ? 1 : 32][3];
 };
 
-// Cooperative over `nthreads` threads (index tid): stages one surface and fills the context.
+// Queries a warp takes at least at a time: enough for a few seeds per lane (by the surface's average
+// number of candidates, SurfDev::seeds), since a warp is busy until its longest seed ends and a refill
+// ends with a pass of the final FP64 steps, as long with one query as with 32; but no more than
+// `spread`, with which the launch has a warp on every scheduler.
+template <int MODE>
+__host__ __device__ inline int least_grab(float seeds, int64_t spread) {
+  const float want = MODE == kModeMixed ? kGrabSeedsMixed : kGrabSeeds64;
+  const int by_seeds = (int)(want / (seeds > 1.0f ? seeds : 1.0f)) + 1;
+  const int k = (int)(spread < 1 ? 1 : (spread < (int64_t)by_seeds ? spread : (int64_t)by_seeds));
+  return k < 32 ? k : 32;
+}
+
+// Where a warp of a persistent launch takes its next queries from: a global counter.  A warp asks
+// for as many queries as it has free slots and gets its share of what is left, or `least`, so that
+// a small launch spreads over all warps and a large one ends with all warps on their last queries.
+struct QueryCounter {
+  unsigned long long* next;
+  int64_t n, seen;
+  float share;  // 1 / resident warps
+  int least;
+  __device__ __forceinline__ int grab(int want, int64_t& q0) {
+    const float fair = (float)(n - seen) * share;
+    int k = fair < (float)want ? (int)fair + 1 : want;
+    k = max(k, least);
+    k = min(k, want);
+    unsigned long long a = 0;
+    if ((threadIdx.x & 31) == 0) a = atomicAdd(next, (unsigned long long)k);
+    q0 = (int64_t)__shfl_sync(0xffffffffu, a, 0);
+    seen = q0 + k;
+    const int64_t left = n - q0;
+    return left < k ? (left > 0 ? (int)left : 0) : k;
+  }
+};
+// A launch's grid: as many warps as take their first queries at once (more would race for them, and
+// leave some schedulers with several warps' queries and others with none), at most the resident ones.
+struct StreamGrid {
+  unsigned blocks;
+  float share;
+  int least;
+};
+template <int MODE>
+inline StreamGrid stream_grid(const SurfDev& s, int64_t n, int64_t resident_ctas) {
+  StreamGrid g;
+  g.least = least_grab<MODE>(s.seeds, n / kSchedulers);
+  const int64_t warps = (n + g.least - 1) / g.least, blocks = (warps + kWarps - 1) / kWarps;
+  g.blocks = (unsigned)(blocks < resident_ctas ? blocks : resident_ctas);
+  g.share = 1.0f / (float)((int64_t)g.blocks * kWarps);
+  return g;
+}
+
+// Cooperative over `nthreads` threads (index tid): stages one surface and its context.
 // The callers synchronise the participating threads before and after.
 template <int KS, int MODE>
-__device__ __forceinline__ void stage_surface(const SurfDev& s, Staged<KS, MODE>& sm, Ctx& cx, int tid, int nthreads) {
+__device__ __forceinline__ void stage_surface(const SurfDev& s, Staged<KS, MODE>& sm, int tid, int nthreads) {
   constexpr int KS64 = Staged<KS, MODE>::KS64;
   const bool smem_tables = s.ns_u <= KS && s.ns_v <= KS;
   const bool smem_tables64 = s.ns_u <= KS64 && s.ns_v <= KS64;
   if (smem_tables) {
-    for (int k = tid; k <= s.ns_u; k += nthreads) {
-      sm.sb32[0][k] = s.bu32[k];
-      if (smem_tables64) sm.sb64[0][k] = s.bu[k];
-      if (k < s.ns_u) {
-        sm.si32[0][k] = s.inv_du32[k];
-        if (smem_tables64) sm.si64[0][k] = s.inv_du[k];
+    for (int dir = 0; dir < 2; ++dir) {
+      const float *b = dir ? s.bv32 : s.bu32, *inv = dir ? s.inv_dv32 : s.inv_du32;
+      const int ns = dir ? s.ns_v : s.ns_u;
+      for (int k = tid; k <= ns; k += nthreads) sm.seg[dir][k] = make_float2(b[k], k < ns ? inv[k] : 0.f);
+      // a bucket's points are right of this value whatever the rounding of their bucket index
+      const float g0 = b[0], gs = (float)KS / (b[ns] - b[0]);
+      for (int i = tid; i < KS; i += nthreads)
+        sm.grid[dir][i] = i == 0 ? 0 : (unsigned char)fast::find_seg(b, ns, g0 + ((float)i - 0.01f) / gs);
+      if (tid == 0) {
+        sm.g0[dir] = g0;
+        sm.gs[dir] = gs;
       }
-    }
-    for (int k = tid; k <= s.ns_v; k += nthreads) {
-      sm.sb32[1][k] = s.bv32[k];
-      if (smem_tables64) sm.sb64[1][k] = s.bv[k];
-      if (k < s.ns_v) {
-        sm.si32[1][k] = s.inv_dv32[k];
-        if (smem_tables64) sm.si64[1][k] = s.inv_dv[k];
+      if (smem_tables64) {
+        const double *b64 = dir ? s.bv : s.bu, *inv64 = dir ? s.inv_dv : s.inv_du;
+        for (int k = tid; k <= ns; k += nthreads) {
+          sm.sb64[dir][k] = b64[k];
+          if (k < ns) sm.si64[dir][k] = inv64[k];
+        }
       }
     }
   }
-  cx.L32 = fast::global_locator<float>(s);
-  cx.L64 = fast::global_locator<double>(s);
-  if (smem_tables) {
-    cx.L32.bu = sm.sb32[0]; cx.L32.bv = sm.sb32[1]; cx.L32.iu = sm.si32[0]; cx.L32.iv = sm.si32[1];
+  if (tid == 0) {
+    Ctx& cx = sm.ctx;
+    sm.fits = smem_tables;
+    cx.L32 = fast::global_locator<float>(s);
+    cx.L64 = fast::global_locator<double>(s);
     if (smem_tables64) {
       cx.L64.bu = sm.sb64[0]; cx.L64.bv = sm.sb64[1]; cx.L64.iu = sm.si64[0]; cx.L64.iv = sm.si64[1];
     }
+    cx.m32 = s.m32;
+    cx.m64 = s.m64;
+    cx.p = s.p;
+    cx.q = s.q;
+    cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
   }
-  cx.m32 = s.m32;
-  cx.m64 = s.m64;
-  cx.p = s.p;
-  cx.q = s.q;
-  cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
   // built nodes are the root alone, or the root and all 64 children (the children of the
   // 2-level tree are built together when the root is divided), so node k keeps index k
   const int nb = s.built[1] ? kTreeNodes : (s.built[0] ? 1 : 0);
@@ -491,287 +646,52 @@ __device__ __forceinline__ void stage_surface(const SurfDev& s, Staged<KS, MODE>
   }
 }
 
-// One warp inverts the queries [q0, min(q0+32, qend)) of the staged surface.
+// One warp inverts the queries that `src` hands out (src.grab), of the staged surface.
+//
+// The warp holds up to 32 queries in slots and its lanes run their (query, seed) pairs.  When the
+// lanes have started every seed of the task list, the slots whose seeds have all ended get their
+// final FP64 steps and results, and new queries take their place while the other slots' last
+// seeds still run: the warp's lanes idle only at the end of the whole launch.  (With chunks of 32
+// queries run to their end one after the other, every chunk ended with a few lanes on its longest
+// seeds, and a launch of fewer than ~32 queries per resident warp left warps without work.)
+// Which lane, slot or warp runs a seed, and when, does not change its arithmetic, and the
+// per-query records do not depend on the order in which seeds end.
+//
 // COUNT: the work-counting variant (nurbs_invert_count): seed iterations and final FP64 polishes
 // are added to counts[0] and counts[1]; the results are the same.
-template <int P, int Q, int MODE, int KS, bool COUNT = false>
-__device__ __forceinline__ void invert_chunk(Staged<KS, MODE>& sm, WarpWork<MODE>& ww, const Ctx& cx,
-                                             const double* __restrict__ Pq,
-                                             int64_t q0, int64_t qend, double* __restrict__ uv_out,
-                                             int* __restrict__ st_out, double* __restrict__ res_out,
-                                             unsigned long long* __restrict__ counts = nullptr) {
+template <int P, int Q, int MODE, int KS, bool COUNT, class Source>
+__device__ __forceinline__ void invert_stream(Staged<KS, MODE>& sm, WarpWork<MODE>& ww, const double* __restrict__ Pq,
+                                              Source& src,
+                                              double* __restrict__ uv_out, int* __restrict__ st_out,
+                                              double* __restrict__ res_out,
+                                              unsigned long long* __restrict__ counts = nullptr) {
+  typedef typename std::conditional<MODE == kModeMixed, float, double>::type T;
+  const Ctx& cx = sm.ctx;
+  const StagedEval<P, Q, KS, MODE> ev{sm};
   unsigned n_iter = 0, n_final = 0;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const int nbl = sm.nb;
-  {
-    const int64_t q = q0 + lane;
-    const bool valid = q < qend;
-    double px = 0, py = 0, pz = 0;
-    if (valid) {
-      px = Pq[3 * q];
-      py = Pq[3 * q + 1];
-      pz = Pq[3 * q + 2];
-    }
-    const float fx = (float)px, fy = (float)py, fz = (float)pz;
-    // ---- cull (exact candidate set, ascending node order).  With f = fl(x) rounded to nearest,
-    // f < rd(lb) implies x < lb and f > ru(lb) implies x > lb (rounding is monotone), so the
-    // FP64 comparison only runs for coordinates within an FP32 ulp of a box face.
-    uint64_t m0 = 0;
-    unsigned m1 = 0;
-    if (valid) {
-      for (int k = 0; k < nbl; ++k) {
-        if (fx >= sm.box32[k][0] && fy >= sm.box32[k][1] && fz >= sm.box32[k][2] && fx <= sm.box32[k][3] &&
-            fy <= sm.box32[k][4] && fz <= sm.box32[k][5]) {
-          const bool surely = fx > sm.box32i[k][0] && fy > sm.box32i[k][1] && fz > sm.box32i[k][2] &&
-                              fx < sm.box32i[k][3] && fy < sm.box32i[k][4] && fz < sm.box32i[k][5];
-          const TreeNodeDev* B = sm.tree + k;
-          if (surely || (px >= B->lb[0] && py >= B->lb[1] && pz >= B->lb[2] && px <= B->rt[0] && py <= B->rt[1] &&
-                         pz <= B->rt[2])) {
-            if (k < 64) m0 |= 1ull << k;
-            else m1 = 1u;
-          }
-        }
-      }
-    }
-    const int cnt = __popcll(m0) + (int)m1;
-    // Task lists.  FP64 schedule: round-major, round r holds seed r of every query with more
-    // than r seeds (rmask[r] = lanes with a seed in round r, rpref[r] = tasks before round r), so
-    // a warp's concurrent seeds come from different queries.  Mixed schedule: lane-major, a
-    // query's seeds consecutive (slpref = exclusive prefix of the candidate counts).
-    const int maxc = __reduce_max_sync(FULL, (unsigned)cnt);
-    int total = 0;
-    for (int r = 0; r < maxc; ++r) {
-      unsigned m = __ballot_sync(FULL, cnt > r);
-      if (MODE != kModeMixed && lane == 0) {
-        ww.srmask[r] = m;
-        ww.srpref[r] = total;
-      }
-      total += __popc(m);
-    }
-    if (MODE != kModeMixed && lane == 0) ww.srpref[maxc] = total;
-    if constexpr (MODE == kModeMixed) {
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += t;
-      }
-      ww.slpref[lane] = incl - cnt;
-    }
-    // the FP32 iterations work relative to the FP32 tables' origin
-    ww.sp32[lane][0] = (float)(px - sm.org[0]);
-    ww.sp32[lane][1] = (float)(py - sm.org[1]);
-    ww.sp32[lane][2] = (float)(pz - sm.org[2]);
-    if constexpr (MODE != kModeMixed) {
-      ww.sp64[lane][0] = px;
-      ww.sp64[lane][1] = py;
-      ww.sp64[lane][2] = pz;
-    }
-    ww.smask0[lane] = m0;
-    ww.smask1[lane] = (unsigned char)m1;
-    if constexpr (MODE == kModeMixed) {
-      Rec32& R = ww.rec[lane];
-      R.d1 = INFINITY;
-      R.d2 = INFINITY;
-      R.de = INFINITY;
-      R.u1 = R.v1 = R.u2 = R.v2 = R.ue = R.ve = 0.f;
-      R.cu1 = R.cv1 = 0;
-    } else {
-      ww.rec[lane].n = 0;
-    }
-    __syncwarp();
+  constexpr int kBatch = MODE == kModeMixed ? kStartBatch : kStartBatch64;
+  constexpr int kRefill = MODE == kModeMixed ? kRefillMixed : kRefill64;
 
-    // decode task t -> (owner lane, node)
-    auto decode = [&](int t, int& ql, int& node) {
-      if constexpr (MODE == kModeMixed) {
-        // lane-major: the largest lane whose exclusive prefix is <= t owns task t (a lane with
-        // no candidates shares its prefix with the next lane and is never the largest)
-        int lo = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (ww.slpref[lo + step] <= t) lo += step;
-        ql = lo;
-        uint64_t mm = ww.smask0[ql];
-        int k = t - ww.slpref[lo];
-        if (k < __popcll(mm)) {
-          node = select_bit(mm, k);
-        } else {
-          node = 64;
-        }
-        return;
-      }
-      // round: the largest r with rpref[r] <= t (rounds are non-empty, so rpref is increasing)
-      int r = 0;
-#pragma unroll
-      for (int step = 64; step > 0; step >>= 1)
-        if (r + step < maxc && ww.srpref[r + step] <= t) r += step;
-      // lane: the (t - rpref[r])-th set bit of rmask[r]
-      const unsigned m = ww.srmask[r];
-      int i = t - ww.srpref[r], pos = 0;
-#pragma unroll
-      for (int w = 16; w > 0; w >>= 1)
-        if (__popc(m & ((1u << (pos + w)) - 1u)) <= i) pos += w;
-      ql = pos;
-      int k = r;  // seed r of that query: its r-th candidate node in ascending order
-      uint64_t mm = ww.smask0[ql];
-      int c0 = __popcll(mm);
-      if (k < c0) {
-        node = select_bit(mm, k);
-      } else {
-        node = 64;
-      }
-    };
+  bool more = true;                    // src may have queries left
+  bool used = false;                   // this lane's slot holds a query
+  int total = 0, next = 0;             // task list: tasks, and how many have been started
+  bool waiting = true;                 // this lane wants a seed (it runs one otherwise)
+  int ql = 0;                          // its slot
+  Seed<T> sd;
+  T tx = 0, ty = 0, tz = 0;
+  int end = kContinue;                 // how its last seed ended, until that is merged
+  T dist = 0;                          // and the squared distance there
 
-    int next = 32;
-    int task = lane;
-    bool active = task < total;
-    int ql = 0, node = 0;
-    if constexpr (MODE == kModeMixed) {
-      Seed<float> sd;
-      float dist = 0.f;
-      float tx = 0, ty = 0, tz = 0;
-      auto start = [&]() {
-        decode(task, ql, node);
-        tx = ww.sp32[ql][0];
-        ty = ww.sp32[ql][1];
-        tz = ww.sp32[ql][2];
-        sd.u = sm.ctr32[node][0];
-        sd.v = sm.ctr32[node][1];
-        sd.prev = INFINITY;
-        sd.it = 0;
-        sd.hu = 0;
-        sd.hv = 0;
-        sd.newton = false;
-        first_step<float>(sm.cd32 + 9 * node, tx, ty, tz, sm.far32, sd);
-      };
-      if (active) start();
-      bool waiting = false;  // finished, waiting for the next batch of starts
-      while (__any_sync(FULL, active || waiting)) {
-        int res = kContinue;
-        if (active) {
-          res = iterate32<P, Q>(cx, tx, ty, tz, sd, dist);
-          if constexpr (COUNT) ++n_iter;
-          if (res == kContinue && !(sd.u >= sm.far32[0] && sd.u <= sm.far32[1] && sd.v >= sm.far32[2] &&
-                                    sd.v <= sm.far32[3]))
-            res = kFailed;
-        }
-        const bool done = active && res != kContinue;
-        const bool keep = res == kConverged && sd.u >= sm.dom32[0] && sd.u <= sm.dom32[1] && sd.v >= sm.dom32[2] &&
-                          sd.v <= sm.dom32[3];
-        // An FP32 minimum within 1 % of the extent outside the domain: near an edge FP32 arithmetic
-        // can end outside while FP64 steps from there reach a minimum inside.  The closest such
-        // result of a query is kept apart and takes the final FP64 steps too when it is close.
-        const bool edge = done && res == kConverged && !keep && sd.u >= sm.near32[0] && sd.u <= sm.near32[1] &&
-                          sd.v >= sm.near32[2] && sd.v <= sm.near32[3];
-        __syncwarp();
-        int cu = 0, cv = 0;
-        bool upd = done && keep;
-        if (upd) {
-          // Records only improve, so a result that cannot change its query's record now never
-          // will: only the others are merged, one lane at a time.
-          cell_of(sm.cell32, sd.u, sd.v, cu, cv);
-          const Rec32& R = ww.rec[ql];
-          if (R.d1 < INFINITY && cu == R.cu1 && cv == R.cv1)
-            upd = before(dist, sd.u, sd.v, R.d1, R.u1, R.v1);
-          else
-            upd = before(dist, sd.u, sd.v, R.d1, R.u1, R.v1) || before(dist, sd.u, sd.v, R.d2, R.u2, R.v2);
-        }
-        const bool upe = edge && before(dist, sd.u, sd.v, ww.rec[ql].de, ww.rec[ql].ue, ww.rec[ql].ve);
-        unsigned fm = __ballot_sync(FULL, upd || upe);
-        while (fm) {
-          int j = __ffs(fm) - 1;
-          if (lane == j) {
-            Rec32& R = ww.rec[ql];
-            if (upd) merge32(R, cu, cv, sd.u, sd.v, dist);
-            else if (before(dist, sd.u, sd.v, R.de, R.ue, R.ve)) { R.ue = sd.u; R.ve = sd.v; R.de = dist; }
-          }
-          __syncwarp();
-          fm &= fm - 1;
-        }
-        if (done) {
-          active = false;
-          waiting = true;
-        }
-        const unsigned wm = __ballot_sync(FULL, waiting);
-        if (wm && (__popc(wm) >= kStartBatch || !__any_sync(FULL, active))) {
-          if (waiting) {
-            task = next + __popc(wm & lt_mask);
-            active = task < total;
-            waiting = false;
-            if (active) start();
-          }
-          next += __popc(wm);
-        }
-      }
-    } else {
-      Seed<double> sd;
-      double tx = 0, ty = 0, tz = 0;
-      auto start = [&]() {
-        decode(task, ql, node);
-        tx = ww.sp64[ql][0];
-        ty = ww.sp64[ql][1];
-        tz = ww.sp64[ql][2];
-        sd.u = sm.ctr[node][0];
-        sd.v = sm.ctr[node][1];
-        sd.prev = INFINITY;
-        sd.it = 0;
-        sd.hu = 0;
-        sd.hv = 0;
-        sd.newton = false;
-        first_step<double>(sm.cd64 + 9 * node, tx, ty, tz, sm.far32, sd);
-      };
-      if (active) start();
-      // lanes whose seed has ended wait until kStartBatch64 are free: their results are merged and
-      // their next seeds started together (the first step is as much FP64 work for one lane as for
-      // all)
-      bool waiting = false, keep = false;
-      double rr = 0;
-      while (__any_sync(FULL, active || waiting)) {
-        if (active) {
-          const int res = iterate64<P, Q>(cx, tx, ty, tz, sd, rr);
-          if constexpr (COUNT) ++n_iter;
-          if (res != kContinue) {
-            keep = res == kConverged && in_domain64(cx, sd.u, sd.v, rr);
-            active = false;
-            waiting = true;
-          }
-        }
-        const unsigned wm = __ballot_sync(FULL, waiting);
-        if (wm && (__popc(wm) >= kStartBatch64 || !__any_sync(FULL, active))) {
-          int cu = 0, cv = 0;
-          if (waiting && keep) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
-          unsigned fm = __ballot_sync(FULL, waiting && keep);
-          while (fm) {
-            int j = __ffs(fm) - 1;
-            if (lane == j) merge64(ww.rec[ql], cu, cv, sd.u, sd.v, rr);
-            __syncwarp();
-            fm &= fm - 1;
-          }
-          if (waiting) {
-            task = next + __popc(wm & lt_mask);
-            active = task < total;
-            waiting = false;
-            keep = false;
-            if (active) start();
-          }
-          next += __popc(wm);
-        }
-      }
-    }
-    __syncwarp();
-
-    // ---- per query: final FP64 steps (MIXED) and the result
+  // this lane's slot: the final FP64 steps (MIXED) and the result of its query
+  auto finish_query = [&]() {
+    const int64_t q = ww.sq[lane];
     int status;
     double ou = __longlong_as_double(0x7ff8000000000000ll), ov = ou, orr = ou;
-    if (cnt == 0) {
-      status = 2;  // NURBS_INV_NO_CANDIDATE
-    } else if constexpr (MODE == kModeMixed) {
-      // the query's FP64 coordinates again (not kept in registers through the seed loop)
-      px = Pq[3 * q];
-      py = Pq[3 * q + 1];
-      pz = Pq[3 * q + 2];
+    if constexpr (MODE == kModeMixed) {
+      const double px = Pq[3 * q], py = Pq[3 * q + 1], pz = Pq[3 * q + 2];
       double us[3], vs[3], rs[3];
       int ns = 0;
       // FP64 minima reached from the records; two within kDistinct are one minimum (split by a
@@ -792,24 +712,28 @@ __device__ __forceinline__ void invert_chunk(Staged<KS, MODE>& sm, WarpWork<MODE
         // minimum's distance); one next to the best is the same minimum split by a cell boundary.
         // The edge record takes them when it is within the same margin.
         const float e1 = sqrtf(dbest) * (1.0f + kPolishMargin) + 1e-5f;
-        if (R.d1 < INFINITY) {
-          const bool second =
-              R.d2 < INFINITY && !(fabsf(R.u2 - R.u1) <= kDistinct32 && fabsf(R.v2 - R.v1) <= kDistinct32);
-          const bool tie = second && R.d2 <= e1 * e1;
-          double u = R.u1, v = R.v1, r;
-          const bool ok1 = final64<P, Q>(cx, px, py, pz, u, v, r);
-          if constexpr (COUNT) ++n_final;
-          if (ok1) add(u, v, r);
-          if (ok1 ? tie : second) {
-            double u2 = R.u2, v2 = R.v2, r2;
+        const bool first = R.d1 < INFINITY;
+        const bool second =
+            first && R.d2 < INFINITY && !(fabsf(R.u2 - R.u1) <= kDistinct32 && fabsf(R.v2 - R.v1) <= kDistinct32);
+        const bool tie = second && R.d2 <= e1 * e1, edge = R.de <= e1 * e1;
+        // One loop over the lane's candidates, the next one taken up in the very iteration after the
+        // last one's end: the warp's steps are the longest sum over a lane's candidates, not the sum
+        // of the longest of the best, of the runners-up and of the edge records.
+        int cand = first ? 0 : 2;
+        Final f;
+        final_start(ev, first ? R.u1 : R.ue, first ? R.v1 : R.ve, f);
+        if constexpr (COUNT) ++n_final;
+        while (cand < 3) {
+          double r;
+          const int end = final_step<P, Q>(cx, ev, px, py, pz, f, r);
+          if (end == kContinue) continue;
+          if (end == kConverged) add(f.u, f.v, r);
+          const bool more2 = cand == 0 && (end == kConverged ? tie : second);
+          cand = more2 ? 1 : (cand < 2 && edge ? 2 : 3);
+          if (cand < 3) {
+            final_start(ev, more2 ? R.u2 : R.ue, more2 ? R.v2 : R.ve, f);
             if constexpr (COUNT) ++n_final;
-            if (final64<P, Q>(cx, px, py, pz, u2, v2, r2)) add(u2, v2, r2);
           }
-        }
-        if (R.de <= e1 * e1) {
-          double u3 = R.ue, v3 = R.ve, r3;
-          if constexpr (COUNT) ++n_final;
-          if (final64<P, Q>(cx, px, py, pz, u3, v3, r3)) add(u3, v3, r3);
         }
       }
       status = ns == 0 ? 3 : finish_status(us, vs, rs, ns, kDistinct, kDistinct, ou, ov, orr);
@@ -819,13 +743,218 @@ __device__ __forceinline__ void invert_chunk(Staged<KS, MODE>& sm, WarpWork<MODE
       for (int k = 0; k < kSols; ++k) rs[k] = k < R.n ? sqrt(R.r[k]) : 0.0;
       status = R.n == 0 ? 3 : finish_status(R.u, R.v, rs, R.n, 2.0 / sm.cell64.iu, 2.0 / sm.cell64.iv, ou, ov, orr);
     }
-    if (valid) {
-      uv_out[2 * q] = ou;
-      uv_out[2 * q + 1] = ov;
-      st_out[q] = status;
-      res_out[q] = orr;
+    uv_out[2 * q] = ou;
+    uv_out[2 * q + 1] = ov;
+    st_out[q] = status;
+    res_out[q] = orr;
+  };
+
+  // A new query for this lane's slot: its candidates and an empty record.  Returns the number of
+  // candidates; a query without any is answered at once.
+  auto load_query = [&](int64_t q) {
+    const double px = Pq[3 * q], py = Pq[3 * q + 1], pz = Pq[3 * q + 2];
+    const float fx = (float)px, fy = (float)py, fz = (float)pz;
+    // ---- cull (exact candidate set, ascending node order).  With f = fl(x) rounded to nearest,
+    // f < rd(lb) implies x < lb and f > ru(lb) implies x > lb (rounding is monotone), so the
+    // FP64 comparison only runs for coordinates within an FP32 ulp of a box face.
+    uint64_t m0 = 0;
+    unsigned m1 = 0;
+    const int nbl = sm.nb;
+    for (int k = 0; k < nbl; ++k) {
+      if (fx >= sm.box32[k][0] && fy >= sm.box32[k][1] && fz >= sm.box32[k][2] && fx <= sm.box32[k][3] &&
+          fy <= sm.box32[k][4] && fz <= sm.box32[k][5]) {
+        const bool surely = fx > sm.box32i[k][0] && fy > sm.box32i[k][1] && fz > sm.box32i[k][2] &&
+                            fx < sm.box32i[k][3] && fy < sm.box32i[k][4] && fz < sm.box32i[k][5];
+        const TreeNodeDev* B = sm.tree + k;
+        if (surely || (px >= B->lb[0] && py >= B->lb[1] && pz >= B->lb[2] && px <= B->rt[0] && py <= B->rt[1] &&
+                       pz <= B->rt[2])) {
+          if (k < 64) m0 |= 1ull << k;
+          else m1 = 1u;
+        }
+      }
     }
+    const int cnt = __popcll(m0) + (int)m1;
+    if (cnt == 0) {
+      const double nan = __longlong_as_double(0x7ff8000000000000ll);
+      uv_out[2 * q] = nan;
+      uv_out[2 * q + 1] = nan;
+      st_out[q] = 2;  // NURBS_INV_NO_CANDIDATE
+      res_out[q] = nan;
+      return 0;
+    }
+    ww.sq[lane] = q;
+    ww.smask0[lane] = m0;
+    ww.sleft[lane] = cnt;
+    if constexpr (MODE == kModeMixed) {
+      // the FP32 iterations work relative to the FP32 tables' origin
+      ww.sp32[lane][0] = (float)(px - sm.org[0]);
+      ww.sp32[lane][1] = (float)(py - sm.org[1]);
+      ww.sp32[lane][2] = (float)(pz - sm.org[2]);
+      Rec32& R = ww.rec[lane];
+      R.d1 = INFINITY;
+      R.d2 = INFINITY;
+      R.de = INFINITY;
+      R.u1 = R.v1 = R.u2 = R.v2 = R.ue = R.ve = 0.f;
+      R.cu1 = R.cv1 = 0;
+    } else {
+      ww.sp64[lane][0] = px;
+      ww.sp64[lane][1] = py;
+      ww.sp64[lane][2] = pz;
+      ww.rec[lane].n = 0;
+    }
+    return cnt;
+  };
+
+  // Finishes the slots whose seeds have all ended, fills the free slots with new queries and lists
+  // their tasks, a query's seeds consecutive in ascending node order.  When src has no queries left
+  // the finished slots wait for the last ones (`last`): one pass of the final steps for all of them.
+  auto refill = [&](bool last) {
+    const bool ended = used && ww.sleft[lane] == 0;
+    const unsigned fm = __ballot_sync(FULL, !used || ended);
+    int64_t q0 = 0;
+    int k = 0;
+    if (more) {
+      k = src.grab(__popc(fm), q0);
+      more = k > 0;
+    }
+    if (ended && (more || last)) {
+      finish_query();
+      used = false;
+    }
+    int cnt = 0;
+    const int r = __popc(fm & lt_mask);
+    if (!used && r < k) {
+      cnt = load_query(q0 + r);
+      used = cnt > 0;
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += t;
+    }
+    ww.slpref[lane] = incl - cnt;
+    total = __shfl_sync(FULL, incl, 31);
+    next = 0;
     __syncwarp();
+  };
+
+  // starts task t: its slot is the largest lane whose exclusive prefix is <= t (a lane without
+  // tasks shares its prefix with the next lane and is never the largest)
+  auto start = [&](int t) {
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (ww.slpref[lo + step] <= t) lo += step;
+    ql = lo;
+    const uint64_t mm = ww.smask0[ql];
+    const int k = t - ww.slpref[lo];
+    const int node = k < __popcll(mm) ? select_bit(mm, k) : 64;
+    if constexpr (MODE == kModeMixed) {
+      tx = ww.sp32[ql][0];
+      ty = ww.sp32[ql][1];
+      tz = ww.sp32[ql][2];
+      sd.u = sm.ctr32[node][0];
+      sd.v = sm.ctr32[node][1];
+    } else {
+      tx = ww.sp64[ql][0];
+      ty = ww.sp64[ql][1];
+      tz = ww.sp64[ql][2];
+      sd.u = sm.ctr[node][0];
+      sd.v = sm.ctr[node][1];
+    }
+    sd.prev = INFINITY;
+    sd.it = 0;
+    sd.hu = 0;
+    sd.hv = 0;
+    sd.newton = false;
+    if constexpr (MODE == kModeMixed) first_step<float>(sm.cd32 + 9 * node, tx, ty, tz, sm.far32, sd);
+    else first_step<double>(sm.cd64 + 9 * node, tx, ty, tz, sm.far32, sd);
+  };
+
+  bool none = true;  // no lane runs a seed
+  for (;;) {
+    refill(none);
+    if (total == 0 && !more && !__any_sync(FULL, used)) break;
+    // ---- seeds, until the lanes that want one find the list exhausted and enough slots are done
+    for (;;) {
+      const unsigned wm = __ballot_sync(FULL, waiting);
+      none = wm == FULL;
+      if (__popc(wm) >= kBatch || none) {
+        // ---- the ended seeds' results, and the next seeds
+        if (end != kContinue) atomicSub(&ww.sleft[ql], 1);
+        int cu = 0, cv = 0;
+        bool upd, edge = false;
+        if constexpr (MODE == kModeMixed) {
+          upd = end == kConverged && sd.u >= sm.dom32[0] && sd.u <= sm.dom32[1] && sd.v >= sm.dom32[2] &&
+                sd.v <= sm.dom32[3];
+          // An FP32 minimum within 1 % of the extent outside the domain: near an edge FP32 arithmetic
+          // can end outside while FP64 steps from there reach a minimum inside.  The closest such
+          // result of a query is kept apart and takes the final FP64 steps too when it is close.
+          edge = end == kConverged && !upd && sd.u >= sm.near32[0] && sd.u <= sm.near32[1] && sd.v >= sm.near32[2] &&
+                 sd.v <= sm.near32[3];
+          if (upd) {
+            // Records only improve, so a result that cannot change its query's record now never
+            // will: only the others are merged, one lane at a time.
+            cell_of(sm.cell32, sd.u, sd.v, cu, cv);
+            const Rec32& R = ww.rec[ql];
+            if (R.d1 < INFINITY && cu == R.cu1 && cv == R.cv1)
+              upd = before(dist, sd.u, sd.v, R.d1, R.u1, R.v1);
+            else
+              upd = before(dist, sd.u, sd.v, R.d1, R.u1, R.v1) || before(dist, sd.u, sd.v, R.d2, R.u2, R.v2);
+          }
+          edge = edge && before(dist, sd.u, sd.v, ww.rec[ql].de, ww.rec[ql].ue, ww.rec[ql].ve);
+        } else {
+          upd = end == kConverged && in_domain64(cx, sd.u, sd.v, dist);
+          if (upd) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
+        }
+        unsigned fm = __ballot_sync(FULL, upd || edge);
+        while (fm) {
+          const int j = __ffs(fm) - 1;
+          if (lane == j) {
+            if constexpr (MODE == kModeMixed) {
+              Rec32& R = ww.rec[ql];
+              if (upd) merge32(R, cu, cv, sd.u, sd.v, dist);
+              else if (before(dist, sd.u, sd.v, R.de, R.ue, R.ve)) { R.ue = sd.u; R.ve = sd.v; R.de = dist; }
+            } else {
+              merge64(ww.rec[ql], cu, cv, sd.u, sd.v, dist);
+            }
+          }
+          __syncwarp();
+          fm &= fm - 1;
+        }
+        end = kContinue;
+        __syncwarp();
+        if (next < total) {
+          const int t = next + __popc(wm & lt_mask);
+          if (waiting && t < total) {
+            waiting = false;
+            start(t);
+          }
+          next += __popc(wm);
+        } else {
+          if (none) break;
+          if (more && __popc(__ballot_sync(FULL, !used || ww.sleft[lane] == 0)) >= kRefill) break;
+        }
+      }
+      if (!waiting) {
+        int res;
+        if constexpr (MODE == kModeMixed) {
+          res = iterate32(ev, tx, ty, tz, sd, dist);
+          if (res == kContinue &&
+              !(sd.u >= sm.far32[0] && sd.u <= sm.far32[1] && sd.v >= sm.far32[2] && sd.v <= sm.far32[3]))
+            res = kFailed;
+        } else {
+          res = iterate64<P, Q>(cx, tx, ty, tz, sd, dist);
+        }
+        if constexpr (COUNT) ++n_iter;
+        if (res != kContinue) {
+          end = res;
+          waiting = true;
+        }
+      }
+      __syncwarp();
+    }
   }
   if constexpr (COUNT) {
     unsigned long long a = n_iter, b = n_final;

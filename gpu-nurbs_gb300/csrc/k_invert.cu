@@ -11,23 +11,27 @@
 //      fixed point is the same stationary point but which converge quadratically;
 //   3. results inside the knot domain are kept; the closest wins.
 //
-// Work distribution.  The grid is persistent (as many CTAs as fit on the GPU at once) and each
-// warp takes chunks of consecutive queries from a global counter until none are left, so
-// warps that drew expensive queries do not hold up the end of the launch.  Chunks hold 32
-// queries; on large launches the last two rounds hold 8, which shortens the tail in which the
-// last warps finish while the others idle.  A query has anywhere from 0 to 65 candidate seeds
-// and a seed needs from 2 to 24 iterations, so one thread per query leaves most lanes of a warp
-// idle.  Each warp flattens its chunk's (query, seed) pairs into a task list (warp prefix sum
-// over the candidate counts) and lanes pull the next tasks as their seeds converge or fail, so
-// all 32 lanes iterate until the warp's list is exhausted, in batches of a few free lanes (the
-// start is divergent work, cheaper done once for several lanes than every iteration for the two or
-// three that just finished).  Finished
-// seeds are merged
-// into per-query records in shared memory (only results that can change a record, one lane at
-// a time).  Every seed runs to its own end (convergence, failure, the iteration cap, or an FP32
-// iterate two domain extents outside the domain), decided by the seed alone, so a query's result
-// does not depend on which other queries share its warp: results are the same alone and in any
-// batch.
+// Work distribution.  A query has anywhere from 0 to 65 candidate seeds and a seed needs from 2 to 24
+// iterations, so one thread per query leaves most lanes of a warp idle.  The grid is persistent (as
+// many CTAs as fit, fewer for small launches); each warp holds up to 32 queries in slots, flattens
+// their (query, seed) pairs into a task list, and its lanes pull the next tasks as their seeds
+// converge or fail, in batches of a few free lanes (the start and the merge of results are divergent
+// work, cheaper done once for several lanes than every iteration for the two or three that just
+// finished).  When the list runs out, the finished queries leave and new ones from a global counter
+// take their slots while the last seeds of the others still run, so a warp's lanes idle only at the
+// end of the launch.  A warp takes its share of what is left of the launch, and at least queries for
+// a few seeds per lane (invert_core.cuh: least_grab).
+//
+// Against chunks of 32 queries run to their end one after the other (with the lookup grid of the
+// staged breakpoints and the merges in batches; us, before and after):
+//   64x64 surface, mixed   1,500 queries  671 -> 147;   20,000  812 -> 480;   2^20  9051 -> 8230
+//   8x8 surface, mixed     1,500 queries  107 ->  73;   60,000  133 -> 122;   2^20  1365 -> 1250
+//   64x64 surface, FP64    2,000 queries 3245 -> 820;   50,021  7390 -> 6670
+//   quintic 256x256        20,000 queries 1212 -> 872;  300,007 6370 -> 5630
+//
+// Every seed runs to its own end (convergence, failure, the iteration cap, or an FP32 iterate two
+// domain extents outside the domain), decided by the seed alone, so a query's result does not depend
+// on which other queries share its warp: results are the same alone and in any batch.
 //
 // Precision schedules (template MODE):
 //   FP64  — every evaluation, solve and update in FP64.  Bound by the FP64 pipe, which a warp's
@@ -51,73 +55,56 @@ namespace {
 
 using namespace inv;
 
-// Register budget: 6 CTAs per SM (80 registers) for the mixed kernel of degrees up to 3; degree 5
-// keeps 128 registers (4 CTAs per SM), its larger Horner state spilling at 80.
-template <int P, int Q, int MODE>
-__global__ void __launch_bounds__(kThreads, MODE == kModeMixed ? ((P == 5 || Q == 5) ? 4 : kMinBlocksMixed) : 4)
+// Register budget.  Mixed: 6 CTAs per SM (80 registers, some spills) hide the exploration's latencies
+// best when every warp refills its slots several times; a launch of at most one slot set per warp of
+// 4 CTAs per SM is bound by the latency of its seeds, and spills lengthen that (64x64 surface, 6 / 4
+// CTAs: 6,000 queries 230 / 204 us, 60,000 835 / 789 us, 2^18 2457 / 2505 us, 2^20 8.26 / 8.63 ms).
+// Degree 5 and the run-time-degree variant keep 128 registers (4 CTAs per SM): their larger Horner
+// state spills heavily at 80.
+template <int P, int Q, int MODE, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS)
     k_invert(SurfDev s, const double* __restrict__ Pq, int64_t n, double* __restrict__ uv_out,
-             int* __restrict__ st_out, double* __restrict__ res_out, unsigned* __restrict__ counter,
-             int64_t n_big) {
+             int* __restrict__ st_out, double* __restrict__ res_out, unsigned long long* __restrict__ counter,
+             StreamGrid grid) {
   __shared__ Staged<kSmemSpans, MODE> sm;           // one surface for the whole CTA
   __shared__ WarpWork<MODE> ww[kWarps];
-  Ctx cx;
-  stage_surface<kSmemSpans>(s, sm, cx, threadIdx.x, blockDim.x);
+  stage_surface<kSmemSpans>(s, sm, threadIdx.x, blockDim.x);
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  // queries [0, n_big) in chunks of 32, then [n_big, n) in chunks of 8
-  const int64_t big = n_big / 32, units = big + (n - n_big + 7) / 8;
-  for (;;) {
-    unsigned ch = 0;
-    if ((threadIdx.x & 31) == 0) ch = atomicAdd(counter, 1u);
-    ch = __shfl_sync(0xffffffffu, ch, 0);
-    if ((int64_t)ch >= units) break;
-    const int64_t q0 = (int64_t)ch < big ? (int64_t)ch * 32 : n_big + ((int64_t)ch - big) * 8;
-    const int64_t q1 = (int64_t)ch < big ? q0 + 32 : min(q0 + 8, n);
-    invert_chunk<P, Q, MODE, kSmemSpans>(sm, ww[warp], cx, Pq, q0, q1, uv_out, st_out, res_out);
-  }
+  QueryCounter src{counter, n, 0, grid.share, grid.least};
+  invert_stream<P, Q, MODE, kSmemSpans, false>(sm, ww[threadIdx.x >> 5], Pq, src, uv_out, st_out, res_out);
 }
 
-// The work-counting variant: the same per-query computation, 32-query chunks from the counter,
-// FP32/FP64 seed iterations and final FP64 polishes added to counts[0..1].  Diagnostic only.
+// The work-counting variant: the same per-query computation, FP32/FP64 seed iterations and final
+// FP64 polishes added to counts[0..1].  Diagnostic only.
 template <int P, int Q, int MODE>
 __global__ void __launch_bounds__(kThreads, 4)
     k_invert_count(SurfDev s, const double* __restrict__ Pq, int64_t n, double* __restrict__ uv_out,
-                   int* __restrict__ st_out, double* __restrict__ res_out, unsigned* __restrict__ counter,
-                   unsigned long long* __restrict__ counts) {
+                   int* __restrict__ st_out, double* __restrict__ res_out, unsigned long long* __restrict__ counter,
+                   StreamGrid grid, unsigned long long* __restrict__ counts) {
   __shared__ Staged<kSmemSpans, MODE> sm;
   __shared__ WarpWork<MODE> ww[kWarps];
-  Ctx cx;
-  stage_surface<kSmemSpans>(s, sm, cx, threadIdx.x, blockDim.x);
+  stage_surface<kSmemSpans>(s, sm, threadIdx.x, blockDim.x);
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  const int64_t units = (n + 31) / 32;
-  for (;;) {
-    unsigned ch = 0;
-    if ((threadIdx.x & 31) == 0) ch = atomicAdd(counter, 1u);
-    ch = __shfl_sync(0xffffffffu, ch, 0);
-    if ((int64_t)ch >= units) break;
-    const int64_t q0 = (int64_t)ch * 32;
-    invert_chunk<P, Q, MODE, kSmemSpans, true>(sm, ww[warp], cx, Pq, q0, min(q0 + 32, n), uv_out, st_out, res_out,
-                                               counts);
-  }
+  QueryCounter src{counter, n, 0, grid.share, grid.least};
+  invert_stream<P, Q, MODE, kSmemSpans, true>(sm, ww[threadIdx.x >> 5], Pq, src, uv_out, st_out, res_out, counts);
 }
 
 template <int P, int Q, int MODE>
 cudaError_t launch_count_mode(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
-                              unsigned* counter, unsigned long long* counts, cudaStream_t st) {
+                              unsigned long long* counter, unsigned long long* counts, cudaStream_t st) {
   if ((n + 31) / 32 > 0x3fffffffLL) return cudaErrorInvalidValue;
   int sms = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t blocks = std::min<int64_t>((n + 32 * kWarps - 1) / (32 * kWarps), (int64_t)(sms > 0 ? sms : 1) * 4);
-  k_invert_count<P, Q, MODE><<<(unsigned)blocks, kThreads, 0, st>>>(s, P_, n, uv, st_, res, counter, counts);
+  const StreamGrid g = stream_grid<MODE>(s, n, (int64_t)(sms > 0 ? sms : 1) * 4);
+  k_invert_count<P, Q, MODE><<<g.blocks, kThreads, 0, st>>>(s, P_, n, uv, st_, res, counter, g, counts);
   return cudaGetLastError();
 }
 
 template <int P, int Q>
 cudaError_t launch_count_pq(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
-                            int prec, unsigned* counter, unsigned long long* counts, cudaStream_t st) {
+                            int prec, unsigned long long* counter, unsigned long long* counts, cudaStream_t st) {
   if (prec == 1) return launch_count_mode<P, Q, kModeMixed>(s, P_, n, uv, st_, res, counter, counts, st);
   return launch_count_mode<P, Q, kModeFP64>(s, P_, n, uv, st_, res, counter, counts, st);
 }
@@ -138,34 +125,39 @@ int64_t resident_ctas(K kernel) {
   return cached[dev];
 }
 
+template <int P, int Q, int MODE, int CTAS>
+cudaError_t launch_budget(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
+                          unsigned long long* counter, cudaStream_t st) {
+  const StreamGrid g = stream_grid<MODE>(s, n, resident_ctas(k_invert<P, Q, MODE, CTAS>));
+  k_invert<P, Q, MODE, CTAS><<<g.blocks, kThreads, 0, st>>>(s, P_, n, uv, st_, res, counter, g);
+  return cudaGetLastError();
+}
+
 template <int P, int Q, int MODE>
 cudaError_t launch_mode(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
-                        unsigned* counter, cudaStream_t st) {
-  const int64_t chunks = (n + 31) / 32;
-  if (chunks > 0x3fffffffLL) return cudaErrorInvalidValue;  // chunk ids are 32-bit
-  int64_t blocks = (chunks + kWarps - 1) / kWarps;
-  const int64_t cap = resident_ctas(k_invert<P, Q, MODE>);
-  if (blocks > cap) blocks = cap;
-  // small chunks for the last two rounds of warps, when there are at least four rounds
-  const int64_t warps = cap * kWarps, tail = 2 * warps * 8;
-  const int64_t n_big = ((n >= 4 * warps * 32 ? n - tail : n) / 32) * 32;  // a multiple of 32
-  k_invert<P, Q, MODE><<<(unsigned)blocks, kThreads, 0, st>>>(s, P_, n, uv, st_, res, counter, n_big);
-  return cudaGetLastError();
+                        unsigned long long* counter, cudaStream_t st) {
+  if ((n + 31) / 32 > 0x3fffffffLL) return cudaErrorInvalidValue;
+  if constexpr (MODE == kModeMixed && (P == 2 || P == 3)) {
+    if (n > (int64_t)32 * 4 * kWarps * kSchedulers / 4)
+      return launch_budget<P, Q, MODE, 6>(s, P_, n, uv, st_, res, counter, st);
+  }
+  return launch_budget<P, Q, MODE, 4>(s, P_, n, uv, st_, res, counter, st);
 }
 
 template <int P, int Q>
 cudaError_t launch_pq(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res, int prec,
-                      unsigned* counter, cudaStream_t st) {
+                      unsigned long long* counter, cudaStream_t st) {
   if (prec == 1) return launch_mode<P, Q, kModeMixed>(s, P_, n, uv, st_, res, counter, st);
   return launch_mode<P, Q, kModeFP64>(s, P_, n, uv, st_, res, counter, st);
 }
 
 // S, Su, Sv at the uv-centre of every built node, FP32 and FP64: the first iteration of every
 // seed starts there, and its evaluation does not depend on the query.  Computed with the same
-// device functions and arguments as the seed iterations, so the values are the same bits.
+// device functions and arguments as the seed iterations, so the values are the same bits.  Then the
+// average number of candidate nodes of these points, by which the inversion sizes its work
+// (cd32[9 * kTreeNodes]).  96 threads.
 template <int P, int Q>
-__device__ void centre_ders(const SurfDev& s, int k) {
-  if (k >= kTreeNodes || !s.built[k]) return;
+__device__ __forceinline__ void centre_of(const SurfDev& s, int k, int& hits) {
   const TreeNodeDev& T = s.tree[k];
   const double cu = (T.uv_lb[0] + T.uv_rt[0]) / 2, cv = (T.uv_lb[1] + T.uv_rt[1]) / 2;  // kernel.cu:154
   const fast::Locator<float> L32 = fast::global_locator<float>(s);
@@ -180,6 +172,28 @@ __device__ void centre_ders(const SurfDev& s, int k) {
     s.cd32[9 * k + c] = f[c];
     s.cd64[9 * k + c] = g[c];
   }
+  const long long x = fast::order_key(g[0]), y = fast::order_key(g[1]), z = fast::order_key(g[2]);
+  for (int j = 0; j < kTreeNodes; ++j) {
+    const TreeNodeDev& B = s.tree[j];
+    if (s.built[j] && x >= fast::order_key(B.lb[0]) && x <= fast::order_key(B.rt[0]) &&
+        y >= fast::order_key(B.lb[1]) && y <= fast::order_key(B.rt[1]) && z >= fast::order_key(B.lb[2]) &&
+        z <= fast::order_key(B.rt[2]))
+      ++hits;
+  }
+}
+template <int P, int Q>
+__device__ void centre_ders(const SurfDev& s, int k) {
+  __shared__ int s_hits, s_built;
+  if (k == 0) s_hits = s_built = 0;
+  __syncthreads();
+  if (k < kTreeNodes && s.built[k]) {
+    int hits = 0;
+    centre_of<P, Q>(s, k, hits);
+    atomicAdd(&s_hits, hits);
+    atomicAdd(&s_built, 1);
+  }
+  __syncthreads();
+  if (k == 0) s.cd32[9 * kTreeNodes] = (float)s_hits / (float)(s_built > 0 ? s_built : 1);
 }
 
 template <int P, int Q>
@@ -214,7 +228,7 @@ cudaError_t launch_centre_ders_batched(const SurfDev* table, const int* ids, int
 }
 
 cudaError_t launch_invert_count(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
-                                double* residual, int precision, unsigned* counter, unsigned long long* counts,
+                                double* residual, int precision, unsigned long long* counter, unsigned long long* counts,
                                 cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (s.p == 3 && s.q == 3) return launch_count_pq<3, 3>(s, P, n, uv, status, residual, precision, counter, counts, st);
@@ -223,7 +237,7 @@ cudaError_t launch_invert_count(const SurfDev& s, const double* P, int64_t n, do
 }
 
 cudaError_t launch_invert(const SurfDev& s, const double* P, int64_t n, double* uv, int* status, double* residual,
-                          int precision, unsigned* counter, cudaStream_t st) {
+                          int precision, unsigned long long* counter, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (s.p == 3 && s.q == 3) return launch_pq<3, 3>(s, P, n, uv, status, residual, precision, counter, st);
   if (s.p == 5 && s.q == 5) return launch_pq<5, 5>(s, P, n, uv, status, residual, precision, counter, st);

@@ -75,10 +75,10 @@ constexpr float kTolMove32 = 1e-6f;    // mixed: an FP32 move this small ends th
 
 // One FP32 projected Newton iteration of the mixed schedule's exploration (the FP64 rules, the
 // point and the tables relative to the control net's centre).  dist2 = |S - P|^2 before the step.
-template <int P, int Q>
-__device__ __forceinline__ int project_iterate32(const Ctx& c, const float dom[4], float px, float py, float pz,
+template <class Eval>
+__device__ __forceinline__ int project_iterate32(const Eval& ev, const float dom[4], float px, float py, float pz,
                                                  PSeed32& sd, float& dist2) {
-  fast::SDer<float> d = fast::eval_at<float, P, Q, 2, true>(c.L32, c.m32, c.p, c.q, sd.u, sd.v, sd.hu, sd.hv);
+  fast::SDer<float> d = ev.template at<2>(sd.u, sd.v, sd.hu, sd.hv);
   const v3<float> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   const float f = dot3(r, r);
   dist2 = f;
@@ -113,7 +113,7 @@ __device__ __forceinline__ int project_iterate32(const Ctx& c, const float dom[4
     float alpha = 1;
     for (int ls = 0;; ++ls) {
       int hu = sd.hu, hv = sd.hv;
-      fast::SDer<float> e = fast::eval_at<float, P, Q, 0, true>(c.L32, c.m32, c.p, c.q, un, vn, hu, hv);
+      fast::SDer<float> e = ev.template at<0>(un, vn, hu, hv);
       const v3<float> rn = {e.S.x - px, e.S.y - py, e.S.z - pz};
       if (dot3(rn, rn) <= f || ls == kMaxHalvings) break;
       alpha *= 0.5f;
@@ -202,15 +202,14 @@ __device__ __forceinline__ int project_iterate(const Ctx& c, double px, double p
 // kPolishSteps, converged at a move <= kTolNewtonProj, the residual from the last step's S, Su, Sv.
 // False when it does not converge: the caller then runs the FP64 schedule's iteration.
 constexpr int kPolishSteps = 8;
-template <int P, int Q>
-__device__ bool project_polish64(const Ctx& c, double px, double py, double pz, double& u, double& v, double& res) {
-  int hu = fast::find_seg_hint(c.L32.bu, c.L32.ns_u, (float)u, 0);
-  int hv = fast::find_seg_hint(c.L32.bv, c.L32.ns_v, (float)v, 0);
+template <int P, int Q, class Eval>
+__device__ bool project_polish64(const Ctx& c, const Eval& ev, double px, double py, double pz, double& u, double& v, double& res) {
+  int hu = 0, hv = 0;
+  ev.spans((float)u, (float)v, hu, hv);
   int hu32 = hu, hv32 = hv;
   for (int it = 0; it < kPolishSteps; ++it) {
     const fast::SDer<double> d = fast::eval_at<double, P, Q, 1>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
-    const fast::SDer<float> e = fast::eval_at<float, P, Q, 2, true>(c.L32, c.m32, c.p, c.q, (float)u, (float)v, hu32,
-                                                                  hv32);
+    const fast::SDer<float> e = ev.template at<2>((float)u, (float)v, hu32, hv32);
     const v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
     const double g0 = dot3(d.Su, r), g1 = dot3(d.Sv, r);
     const double a00 = dot3(d.Su, d.Su), a01 = dot3(d.Su, d.Sv), a11 = dot3(d.Sv, d.Sv);
@@ -253,10 +252,12 @@ __device__ bool project_polish64(const Ctx& c, double px, double py, double pz, 
 // One warp projects the queries [q0, min(q0+32, qend)).
 template <int P, int Q, int MODE>
 __device__ __forceinline__ void project_chunk(const Staged<kSmemSpans, MODE>& sm, const ProjStaged& ps,
-                                              const float* __restrict__ lattice, ProjWarp<MODE>& ww, const Ctx& cx,
+                                              const float* __restrict__ lattice, ProjWarp<MODE>& ww,
                                               const double* __restrict__ Pq, int64_t q0, int64_t qend,
                                               double* __restrict__ uv_out, int* __restrict__ st_out,
                                               double* __restrict__ res_out) {
+  const Ctx& cx = sm.ctx;
+  const StagedEval<P, Q, kSmemSpans, MODE> ev{sm};
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -396,7 +397,7 @@ __device__ __forceinline__ void project_chunk(const Staged<kSmemSpans, MODE>& sm
     bool waiting = false;  // finished, waiting for the next batch of starts (as the inversion's)
     while (__any_sync(FULL, active || waiting)) {
       int res = kContinue;
-      if (active) res = project_iterate32<P, Q>(cx, dom32, tx, ty, tz, sd, dist);
+      if (active) res = project_iterate32(ev, dom32, tx, ty, tz, sd, dist);
       const bool done = active && res != kContinue;
       __syncwarp();
       int cu = 0, cv = 0;
@@ -491,7 +492,7 @@ __device__ __forceinline__ void project_chunk(const Staged<kSmemSpans, MODE>& sm
       sd.hu = 0;
       sd.hv = 0;
       double rr;
-      if (!project_polish64<P, Q>(cx, px, py, pz, sd.u, sd.v, rr)) {
+      if (!project_polish64<P, Q>(cx, ev, px, py, pz, sd.u, sd.v, rr)) {
         sd.u = u0;
         sd.v = v0;
         int r = kContinue;
@@ -544,13 +545,12 @@ struct ProjSmem {
 template <int P, int Q, int MODE>
 __global__ void __launch_bounds__(kThreads, (MODE == kModeMixed && P != 0) ? 5 : 3)
     k_project(SurfDev s, const double* __restrict__ Pq, int64_t n, double* __restrict__ uv_out,
-              int* __restrict__ st_out, double* __restrict__ res_out, unsigned* __restrict__ counter) {
+              int* __restrict__ st_out, double* __restrict__ res_out, unsigned long long* __restrict__ counter) {
   extern __shared__ __align__(16) unsigned char smem[];
   Staged<kSmemSpans, MODE>& sm = *reinterpret_cast<Staged<kSmemSpans, MODE>*>(smem);
   ProjStaged& ps = *reinterpret_cast<ProjStaged*>(smem + ProjSmem<MODE>::ps);
   ProjWarp<MODE>* ww = reinterpret_cast<ProjWarp<MODE>*>(smem + ProjSmem<MODE>::ww);
-  Ctx cx;
-  stage_surface<kSmemSpans>(s, sm, cx, threadIdx.x, blockDim.x);
+  stage_surface<kSmemSpans>(s, sm, threadIdx.x, blockDim.x);
   for (int e = threadIdx.x; e < kTreeNodes * kConeStride; e += blockDim.x)
     ps.cone[e / kConeStride][e % kConeStride] = s.cone[e];
   for (int e = threadIdx.x; e < kTreeNodes * 9; e += blockDim.x) {
@@ -564,18 +564,18 @@ __global__ void __launch_bounds__(kThreads, (MODE == kModeMixed && P != 0) ? 5 :
   const int warp = threadIdx.x >> 5;
   const int64_t units = (n + 31) / 32;
   for (;;) {
-    unsigned ch = 0;
-    if ((threadIdx.x & 31) == 0) ch = atomicAdd(counter, 1u);
+    unsigned long long ch = 0;
+    if ((threadIdx.x & 31) == 0) ch = atomicAdd(counter, 1ull);
     ch = __shfl_sync(0xffffffffu, ch, 0);
     if ((int64_t)ch >= units) break;
     const int64_t q0 = (int64_t)ch * 32;
-    project_chunk<P, Q, MODE>(sm, ps, s.lattice, ww[warp], cx, Pq, q0, min(q0 + 32, n), uv_out, st_out, res_out);
+    project_chunk<P, Q, MODE>(sm, ps, s.lattice, ww[warp], Pq, q0, min(q0 + 32, n), uv_out, st_out, res_out);
   }
 }
 
 template <int P, int Q, int MODE>
 cudaError_t launch_project_mode(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
-                                unsigned* counter, cudaStream_t st) {
+                                unsigned long long* counter, cudaStream_t st) {
   const int64_t chunks = (n + 31) / 32;
   if (chunks > 0x3fffffffLL) return cudaErrorInvalidValue;  // chunk ids are 32-bit
   constexpr size_t bytes = ProjSmem<MODE>::bytes;
@@ -599,7 +599,7 @@ cudaError_t launch_project_mode(const SurfDev& s, const double* P_, int64_t n, d
 
 template <int P, int Q>
 cudaError_t launch_project_pq(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
-                              int precision, unsigned* counter, cudaStream_t st) {
+                              int precision, unsigned long long* counter, cudaStream_t st) {
   if (precision == kModeMixed) return launch_project_mode<P, Q, kModeMixed>(s, P_, n, uv, st_, res, counter, st);
   return launch_project_mode<P, Q, kModeFP64>(s, P_, n, uv, st_, res, counter, st);
 }
@@ -607,7 +607,7 @@ cudaError_t launch_project_pq(const SurfDev& s, const double* P_, int64_t n, dou
 }  // namespace
 
 cudaError_t launch_project(const SurfDev& s, const double* P, int64_t n, double* uv, int* status, double* residual,
-                           int precision, unsigned* counter, cudaStream_t st) {
+                           int precision, unsigned long long* counter, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (s.p == 3 && s.q == 3) return launch_project_pq<3, 3>(s, P, n, uv, status, residual, precision, counter, st);
   if (s.p == 5 && s.q == 5) return launch_project_pq<5, 5>(s, P, n, uv, status, residual, precision, counter, st);

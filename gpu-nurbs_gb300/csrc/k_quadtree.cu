@@ -167,7 +167,7 @@ __device__ bool node_trajectory(const SurfDev& s, const Ctx& cx, double px, doub
     float dist;
     int r = kContinue;
     while (r == kContinue) {
-      r = iterate32<P, Q>(cx, tx, ty, tz, sd, dist);
+      r = iterate32(GlobalEval<P, Q>{cx}, tx, ty, tz, sd, dist);
       if (r == kContinue && !(sd.u >= far[0] && sd.u <= far[1] && sd.v >= far[2] && sd.v <= far[3])) r = kFailed;
     }
     if (r != kConverged) return false;
@@ -342,7 +342,7 @@ template <int P, int Q, int MODE>
 __global__ void __launch_bounds__(kThreads)
     k_invert_quadtree(SurfDev s, const double* __restrict__ qtbox, const double* __restrict__ Pq, int64_t n,
                       double max_edge, double* __restrict__ uv_out, int* __restrict__ st_out,
-                      double* __restrict__ res_out, unsigned* __restrict__ counter) {
+                      double* __restrict__ res_out, unsigned long long* __restrict__ counter) {
   __shared__ QtWarp ww[kWarps];
   Ctx cx;
   cx.L32 = fast::global_locator<float>(s);
@@ -362,8 +362,8 @@ __global__ void __launch_bounds__(kThreads)
   // queries; the warp then searches the rest one by one from the root's split
   const int64_t chunks = (n + 31) / 32;
   for (;;) {
-    unsigned ch = 0;
-    if (lane == 0) ch = atomicAdd(counter, 1u);
+    unsigned long long ch = 0;
+    if (lane == 0) ch = atomicAdd(counter, 1ull);
     ch = __shfl_sync(FULL, ch, 0);
     if ((int64_t)ch >= chunks) break;
     const int64_t qi = (int64_t)ch * 32 + lane;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kThreads)
 
 template <int P, int Q, int MODE>
 cudaError_t launch_quadtree_mode(const SurfDev& s, const double* P_, int64_t n, double max_edge, double* uv, int* st_,
-                                 double* res, unsigned* counter, cudaStream_t st) {
+                                 double* res, unsigned long long* counter, cudaStream_t st) {
   if ((n + 31) / 32 > 0xffffffffLL) return cudaErrorInvalidValue;  // chunk ids are 32-bit
   static int cached[64] = {0};
   int dev = 0;
@@ -426,7 +426,7 @@ cudaError_t launch_quadtree_mode(const SurfDev& s, const double* P_, int64_t n, 
 
 template <int P, int Q>
 cudaError_t launch_quadtree_pq(const SurfDev& s, const double* P_, int64_t n, double max_edge, double* uv, int* st_,
-                               double* res, int precision, unsigned* counter, cudaStream_t st) {
+                               double* res, int precision, unsigned long long* counter, cudaStream_t st) {
   if (precision == kModeMixed)
     return launch_quadtree_mode<P, Q, kModeMixed>(s, P_, n, max_edge, uv, st_, res, counter, st);
   return launch_quadtree_mode<P, Q, kModeFP64>(s, P_, n, max_edge, uv, st_, res, counter, st);
@@ -435,7 +435,7 @@ cudaError_t launch_quadtree_pq(const SurfDev& s, const double* P_, int64_t n, do
 }  // namespace
 
 cudaError_t launch_invert_quadtree(const SurfDev& s, const double* P, int64_t n, double max_edge, double* uv,
-                                   int* status, double* residual, int precision, unsigned* counter, cudaStream_t st) {
+                                   int* status, double* residual, int precision, unsigned long long* counter, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (s.p == 3 && s.q == 3)
     return launch_quadtree_pq<3, 3>(s, P, n, max_edge, uv, status, residual, precision, counter, st);

@@ -37,7 +37,8 @@ constexpr int kConeStride = 20;   // floats per normal-cone record
 //                                    the surface's extent, not by its distance from the origin
 //   tree[65]                         TreeNodeDev; divided[65], built[65]
 //   cd32[65][9], cd64[65][9]         S, Su, Sv at every built node's uv-centre (the inversion seeds),
-//                                    FP32 (relative to org) and FP64, written after the tree
+//                                    FP32 (relative to org) and FP64, written after the tree; then
+//                                    cd32[65*9], the average number of candidates of those points
 //   nbox[65][6]                      normal boxes (lb xyz, rt xyz) of the built nodes
 //   cone[65][kConeStride]            FP32 projection culling record of each built node, relative to
 //                                    org: bound-box ball centre (0..2) and radius (3), normal-cone
@@ -78,6 +79,7 @@ struct SurfDev {
   double* basis_u;        // per-span basis-to-power matrices (conversion scratch kept with the surface)
   double* basis_v;
   float* cd32;            // seed-centre derivatives (see above)
+  float seeds;            // single surfaces: a host copy of cd32[65*9] (0 before the tree is built)
   double* cd64;
   double* nbox;           // normal cones (see above)
   float* cone;
@@ -150,23 +152,23 @@ cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int n
 
 // stage d.  counter: one device word, zero when the launch starts (the kernel's chunk counter).
 cudaError_t launch_invert(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
-                          double* residual, int precision, unsigned* counter, cudaStream_t st);
+                          double* residual, int precision, unsigned long long* counter, cudaStream_t st);
 // p-curves: continuation from the neighbours' pass-1 answers, then flags (k_pcurve.cu)
 cudaError_t launch_pcurve_passes(const SurfDev& s, const double* C, int64_t n, const double* uv0, const int* st0,
                                  const double* res0, double* uv, int* st, double* res, int* flags,
                                  cudaStream_t stream);
 // the projection: closest point over the closed domain (k_project.cu)
 cudaError_t launch_project(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
-                           double* residual, int precision, unsigned* counter, cudaStream_t st);
+                           double* residual, int precision, unsigned long long* counter, cudaStream_t st);
 // adaptive quadtree inversion (k_quadtree.cu)
 cudaError_t launch_invert_quadtree(const SurfDev& s, const double* P, int64_t n, double max_edge, double* uv,
-                                   int* status, double* residual, int precision, unsigned* counter, cudaStream_t st);
+                                   int* status, double* residual, int precision, unsigned long long* counter, cudaStream_t st);
 // S, Su, Sv at the built nodes' uv-centres (cd32/cd64), after the tree is built
 cudaError_t launch_centre_ders(const SurfDev& s, cudaStream_t st);
 cudaError_t launch_centre_ders_batched(const SurfDev* table, const int* ids, int count, cudaStream_t st);
 // the work-counting variant; counts[0] += seed iterations, counts[1] += final FP64 polishes
 cudaError_t launch_invert_count(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
-                                double* residual, int precision, unsigned* counter, unsigned long long* counts,
+                                double* residual, int precision, unsigned long long* counter, unsigned long long* counts,
                                 cudaStream_t st);
 
 }  // namespace gnurbs

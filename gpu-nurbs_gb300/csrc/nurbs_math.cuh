@@ -678,6 +678,16 @@ __device__ __forceinline__ int find_seg_hint(const T* b, int ns, T x, int hint) 
   return lo;
 }
 
+// S and derivatives at local (lu, lv) of span (hu, hv); su, sv = d(local)/d(parameter).
+template <typename T, int P, int Q, int ORDER, bool FAST = false>
+__device__ __forceinline__ SDer<T> eval_span(const T* __restrict__ m, int p, int q, int ns_v, int hu, int hv, T lu, T lv,
+                                             T su, T sv) {
+  const int k12 = sizeof(T) == 4 ? span_coefs32(p, q) : (p + 1) * (q + 1);
+  const T* span = m + (size_t)(hu * ns_v + hv) * k12 * 4;
+  RDer<T> d = span_contract<T, P, Q, ORDER>(span, p, q, lu, lv);
+  return quotient<T, ORDER, FAST>(d, su, sv);
+}
+
 // eval_point with explicit breakpoint tables and span hints (updated in place).
 template <typename T, int P, int Q, int ORDER, bool FAST = false>
 __device__ __forceinline__ SDer<T> eval_at(const Locator<T>& L, const T* __restrict__ m, int p, int q, T u, T v,
@@ -687,10 +697,7 @@ __device__ __forceinline__ SDer<T> eval_at(const Locator<T>& L, const T* __restr
   T idu = L.iu[hu], idv = L.iv[hv];
   T lu = (u - L.bu[hu]) * idu;
   T lv = (v - L.bv[hv]) * idv;
-  const int k12 = sizeof(T) == 4 ? span_coefs32(p, q) : (p + 1) * (q + 1);
-  const T* span = m + (size_t)(hu * L.ns_v + hv) * k12 * 4;
-  RDer<T> d = span_contract<T, P, Q, ORDER>(span, p, q, lu, lv);
-  return quotient<T, ORDER, FAST>(d, L.ru * idu, L.rv * idv);
+  return eval_span<T, P, Q, ORDER, FAST>(m, p, q, L.ns_v, hu, hv, lu, lv, L.ru * idu, L.rv * idv);
 }
 
 }  // namespace fast

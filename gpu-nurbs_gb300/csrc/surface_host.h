@@ -113,7 +113,7 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
   S.o_m32 = take(nspan * (size_t)span_coefs32(p, q) * 4 * 4);
   S.o_bas_u = take((size_t)nsu * (p + 1) * (p + 1) * 8);
   S.o_bas_v = take((size_t)nsv * (q + 1) * (q + 1) * 8);
-  S.o_cd32 = take(kTreeNodes * 9 * 4);
+  S.o_cd32 = take((kTreeNodes * 9 + 1) * 4);
   S.o_cd64 = take(kTreeNodes * 9 * 8);
   S.o_nbox = take(kTreeNodes * 6 * 8);
   S.o_cone = take(kTreeNodes * kConeStride * 4);
