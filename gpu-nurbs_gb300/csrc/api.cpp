@@ -231,7 +231,7 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
   if ((rc = fetch(weights, ncp, ptr_kind, hw, st))) return rc;
   SurfaceHost S;
   std::string err;
-  if ((rc = prepare_surface(p, q, nu, nv, ku.data(), kv.data(), hc.data(), hw.data(), S, err)))
+  if ((rc = prepare_surface(p, q, nu, nv, ku.data(), kv.data(), hc.data(), hw.data(), S, err, true)))
     return fail(rc, "%s", err.c_str());
   nurbs_surface_s* s = new (std::nothrow) nurbs_surface_s();
   if (!s) return fail(NURBS_E_NOMEM, "host allocation failed");

@@ -291,10 +291,10 @@ __device__ __forceinline__ int final_step(const Ctx& c, const Eval& ev, double p
   }
   return ++f.it < kMaxFinal64 ? kContinue : kFailed;
 }
-template <int P, int Q>
-__device__ bool final64(const Ctx& c, double px, double py, double pz, double& u, double& v, double& res) {
+template <int P, int Q, class Eval>
+__device__ __forceinline__ bool final64(const Ctx& c, const Eval& ev, double px, double py, double pz, double& u,
+                                        double& v, double& res) {
   Final f;
-  const GlobalEval<P, Q> ev{c};
   final_start(ev, u, v, f);
   int r = kContinue;
   while (r == kContinue) r = final_step<P, Q>(c, ev, px, py, pz, f, res);
@@ -414,35 +414,17 @@ __device__ __forceinline__ int finish_status(const double* us, const double* vs,
   return 0;
 }
 
-// One surface staged in shared memory: tree boxes (FP32 outward-rounded and exact FP64), seed
-// centres, domain, and breakpoint tables when the surface has at most KS spans per direction.
-// FP64 breakpoint tables are staged only for the FP64 schedule: the mixed schedule reads them in
-// its few final FP64 steps from global memory, which leaves more of the SM's memory to L1.
-template <int KS, int MODE>
-struct Staged {
-  static constexpr int KS64 = MODE == kModeMixed ? 1 : KS;
-  float box32[kTreeNodes][6];   // rounded outward: a point outside is outside the exact box
-  float box32i[kTreeNodes][6];  // rounded inward: a point strictly inside is inside the exact box
-  const TreeNodeDev* tree;     // exact FP64 boxes, read only near a face (global memory, L2)
-  double ctr[kTreeNodes][2];
-  float ctr32[kTreeNodes][2];
-  double org[3];    // origin of the FP32 tables: FP32 iterations see P - org
-  const float* cd32;   // S, Su, Sv at the node centres (FP32, relative to org), 9 per node
-  const double* cd64;  // the same in FP64
-  float dom32[4];
-  float near32[4];  // 1 % of the extent around the domain: FP32 minima here are edge records
-  float far32[4];  // two domain extents around the domain: an FP32 iterate beyond is abandoned
-  Cells<float> cell32;
-  Cells<double> cell64;
-  int nb;
-  Ctx ctx;      // the surface's context: one copy for all threads, its fields read where they are used
-  bool fits;    // breakpoint tables staged (at most KS spans per direction)
+// A surface's context and FP32 breakpoint tables staged in shared memory, when the surface has at
+// most KS spans per direction.
+template <int KS>
+struct SpanTables {
+  Ctx ctx;    // one copy for all threads, its fields read where they are used
+  bool fits;  // breakpoint tables staged
   // FP32 breakpoints and inverse span lengths, and a lookup grid over the domain: KS equal buckets,
   // each with the span of its left end (or one before)
   float2 seg[2][KS + 1];
   float g0[2], gs[2];  // bucket of x: (x - g0) * gs
   unsigned char grid[2][KS];
-  double sb64[2][KS64 + 1], si64[2][KS64];
 
   // The span of x, as find_seg_hint's: two or three dependent shared-memory reads instead of a
   // bisection's 6 to 8 (which the whole warp runs as soon as one lane has left its last span; the
@@ -462,9 +444,65 @@ struct Staged {
   }
 };
 
-template <int P, int Q, int KS, int MODE>
+// Cooperative over `nthreads` threads (index tid); the callers synchronise before and after.
+template <int KS>
+__device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& sm, int tid, int nthreads) {
+  const bool smem_tables = s.ns_u <= KS && s.ns_v <= KS;
+  if (smem_tables) {
+    for (int dir = 0; dir < 2; ++dir) {
+      const float *b = dir ? s.bv32 : s.bu32, *inv = dir ? s.inv_dv32 : s.inv_du32;
+      const int ns = dir ? s.ns_v : s.ns_u;
+      for (int k = tid; k <= ns; k += nthreads) sm.seg[dir][k] = make_float2(b[k], k < ns ? inv[k] : 0.f);
+      // a bucket's points are right of this value whatever the rounding of their bucket index
+      const float g0 = b[0], gs = (float)KS / (b[ns] - b[0]);
+      for (int i = tid; i < KS; i += nthreads)
+        sm.grid[dir][i] = i == 0 ? 0 : (unsigned char)fast::find_seg(b, ns, g0 + ((float)i - 0.01f) / gs);
+      if (tid == 0) {
+        sm.g0[dir] = g0;
+        sm.gs[dir] = gs;
+      }
+    }
+  }
+  if (tid == 0) {
+    Ctx& cx = sm.ctx;
+    sm.fits = smem_tables;
+    cx.L32 = fast::global_locator<float>(s);
+    cx.L64 = fast::global_locator<double>(s);
+    cx.m32 = s.m32;
+    cx.m64 = s.m64;
+    cx.p = s.p;
+    cx.q = s.q;
+    cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
+  }
+}
+
+// One surface staged in shared memory: tree boxes (FP32 outward-rounded and exact FP64), seed
+// centres, domain, and breakpoint tables when the surface has at most KS spans per direction.
+// FP64 breakpoint tables are staged only for the FP64 schedule: the mixed schedule reads them in
+// its few final FP64 steps from global memory, which leaves more of the SM's memory to L1.
+template <int KS, int MODE>
+struct Staged : SpanTables<KS> {
+  static constexpr int KS64 = MODE == kModeMixed ? 1 : KS;
+  float box32[kTreeNodes][6];   // rounded outward: a point outside is outside the exact box
+  float box32i[kTreeNodes][6];  // rounded inward: a point strictly inside is inside the exact box
+  const TreeNodeDev* tree;     // exact FP64 boxes, read only near a face (global memory, L2)
+  double ctr[kTreeNodes][2];
+  float ctr32[kTreeNodes][2];
+  double org[3];    // origin of the FP32 tables: FP32 iterations see P - org
+  const float* cd32;   // S, Su, Sv at the node centres (FP32, relative to org), 9 per node
+  const double* cd64;  // the same in FP64
+  float dom32[4];
+  float near32[4];  // 1 % of the extent around the domain: FP32 minima here are edge records
+  float far32[4];  // two domain extents around the domain: an FP32 iterate beyond is abandoned
+  Cells<float> cell32;
+  Cells<double> cell64;
+  int nb;
+  double sb64[2][KS64 + 1], si64[2][KS64];
+};
+
+template <int P, int Q, int KS>
 struct StagedEval {
-  const Staged<KS, MODE>& sm;
+  const SpanTables<KS>& sm;
   __device__ __forceinline__ void spans(float u, float v, int& hu, int& hv) const {
     if (sm.fits) {
       hu = sm.span(0, sm.ctx.L32.ns_u, u);
@@ -563,43 +601,20 @@ inline StreamGrid stream_grid(const SurfDev& s, int64_t n, int64_t resident_ctas
 template <int KS, int MODE>
 __device__ __forceinline__ void stage_surface(const SurfDev& s, Staged<KS, MODE>& sm, int tid, int nthreads) {
   constexpr int KS64 = Staged<KS, MODE>::KS64;
-  const bool smem_tables = s.ns_u <= KS && s.ns_v <= KS;
-  const bool smem_tables64 = s.ns_u <= KS64 && s.ns_v <= KS64;
-  if (smem_tables) {
+  stage_tables(s, sm, tid, nthreads);
+  if (s.ns_u <= KS64 && s.ns_v <= KS64) {
     for (int dir = 0; dir < 2; ++dir) {
-      const float *b = dir ? s.bv32 : s.bu32, *inv = dir ? s.inv_dv32 : s.inv_du32;
+      const double *b64 = dir ? s.bv : s.bu, *inv64 = dir ? s.inv_dv : s.inv_du;
       const int ns = dir ? s.ns_v : s.ns_u;
-      for (int k = tid; k <= ns; k += nthreads) sm.seg[dir][k] = make_float2(b[k], k < ns ? inv[k] : 0.f);
-      // a bucket's points are right of this value whatever the rounding of their bucket index
-      const float g0 = b[0], gs = (float)KS / (b[ns] - b[0]);
-      for (int i = tid; i < KS; i += nthreads)
-        sm.grid[dir][i] = i == 0 ? 0 : (unsigned char)fast::find_seg(b, ns, g0 + ((float)i - 0.01f) / gs);
-      if (tid == 0) {
-        sm.g0[dir] = g0;
-        sm.gs[dir] = gs;
-      }
-      if (smem_tables64) {
-        const double *b64 = dir ? s.bv : s.bu, *inv64 = dir ? s.inv_dv : s.inv_du;
-        for (int k = tid; k <= ns; k += nthreads) {
-          sm.sb64[dir][k] = b64[k];
-          if (k < ns) sm.si64[dir][k] = inv64[k];
-        }
+      for (int k = tid; k <= ns; k += nthreads) {
+        sm.sb64[dir][k] = b64[k];
+        if (k < ns) sm.si64[dir][k] = inv64[k];
       }
     }
-  }
-  if (tid == 0) {
-    Ctx& cx = sm.ctx;
-    sm.fits = smem_tables;
-    cx.L32 = fast::global_locator<float>(s);
-    cx.L64 = fast::global_locator<double>(s);
-    if (smem_tables64) {
+    if (tid == 0) {
+      Ctx& cx = sm.ctx;
       cx.L64.bu = sm.sb64[0]; cx.L64.bv = sm.sb64[1]; cx.L64.iu = sm.si64[0]; cx.L64.iv = sm.si64[1];
     }
-    cx.m32 = s.m32;
-    cx.m64 = s.m64;
-    cx.p = s.p;
-    cx.q = s.q;
-    cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
   }
   // built nodes are the root alone, or the root and all 64 children (the children of the
   // 2-level tree are built together when the root is divided), so node k keeps index k
@@ -667,7 +682,7 @@ __device__ __forceinline__ void invert_stream(Staged<KS, MODE>& sm, WarpWork<MOD
                                               unsigned long long* __restrict__ counts = nullptr) {
   typedef typename std::conditional<MODE == kModeMixed, float, double>::type T;
   const Ctx& cx = sm.ctx;
-  const StagedEval<P, Q, KS, MODE> ev{sm};
+  const StagedEval<P, Q, KS> ev{sm};
   unsigned n_iter = 0, n_final = 0;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;

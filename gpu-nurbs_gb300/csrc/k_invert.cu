@@ -110,8 +110,8 @@ cudaError_t launch_count_pq(const SurfDev& s, const double* P_, int64_t n, doubl
 }
 
 // CTAs of a kernel that fit on the current GPU at once (queried once per kernel and device).
-template <class K>
-int64_t resident_ctas(K kernel) {
+template <int P, int Q, int MODE, int CTAS>
+int64_t resident_ctas() {
   static int cached[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -119,7 +119,7 @@ int64_t resident_ctas(K kernel) {
   if (!cached[dev]) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_invert<P, Q, MODE, CTAS>, kThreads, 0);
     cached[dev] = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   }
   return cached[dev];
@@ -128,7 +128,7 @@ int64_t resident_ctas(K kernel) {
 template <int P, int Q, int MODE, int CTAS>
 cudaError_t launch_budget(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
                           unsigned long long* counter, cudaStream_t st) {
-  const StreamGrid g = stream_grid<MODE>(s, n, resident_ctas(k_invert<P, Q, MODE, CTAS>));
+  const StreamGrid g = stream_grid<MODE>(s, n, resident_ctas<P, Q, MODE, CTAS>());
   k_invert<P, Q, MODE, CTAS><<<g.blocks, kThreads, 0, st>>>(s, P_, n, uv, st_, res, counter, g);
   return cudaGetLastError();
 }

@@ -48,7 +48,7 @@ template <int P, int Q>
 __device__ bool continue_from(const Ctx& cx, double px, double py, double pz, double& u, double& v, double& res) {
   {
     double uu = u, vv = v;
-    if (final64<P, Q>(cx, px, py, pz, uu, vv, res)) {
+    if (final64<P, Q>(cx, GlobalEval<P, Q>{cx}, px, py, pz, uu, vv, res)) {
       u = uu;
       v = vv;
       return true;

@@ -257,7 +257,7 @@ __device__ __forceinline__ void project_chunk(const Staged<kSmemSpans, MODE>& sm
                                               double* __restrict__ uv_out, int* __restrict__ st_out,
                                               double* __restrict__ res_out) {
   const Ctx& cx = sm.ctx;
-  const StagedEval<P, Q, kSmemSpans, MODE> ev{sm};
+  const StagedEval<P, Q, kSmemSpans> ev{sm};
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt_mask = (1u << lane) - 1u;

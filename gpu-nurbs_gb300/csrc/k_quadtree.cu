@@ -3,25 +3,30 @@
 // control-net boxes (Inverse, src/kernel/kernel.cu:4-104; BoundingBoxCheck :106-149;
 // getSplitType :251-298; NODE_MAX_SIZE 64, src/kernel/kernel.cuh:13).
 //
-// A persistent grid whose warps take chunks of 32 queries from a counter.  The first layer (the
-// root: its precomputed box and one trajectory from the domain's centre) runs lane per query and
-// answers most queries.  A query it leaves open is then searched by the whole warp.  With MODE
-// mixed every node's trajectory runs in FP32 and its end takes FP64 Newton steps (the mixed
-// inversion's final steps); the box checks and split decisions stay exact FP64:
-//   * a layer's nodes live in shared memory; each node's control-point box is reduced by the
-//     whole warp (lanes stride over the node's control-point rows and columns, min/max by
-//     shuffles: exact, so the pass/fail decisions equal the oracle's);
-//   * the passing nodes' trajectories run one per lane (from the node centre); a result counts
-//     when it converged inside the domain within max_edge of P;
-//   * the first layer with a result answers (its closest result; AMBIGUOUS as in the inversion);
-//     otherwise each passing node is split by the reference's getSplitType, decided in FP32 where
-//     its lengths are clearly off max_edge and else evaluated with the reference-order FP64
-//     functions (this translation unit is compiled with --fmad=false, so the split decisions,
-//     and with them the tree, are the oracle's; the v-length uses the v-derivative, which the
-//     reference takes with MatrixSurfaceDerivativeU), and the children are compacted into the
-//     next layer in the reference's order by a warp prefix sum.
-// Culled nodes are not split (their control-point box does not hold P, so neither does their
-// surface); a layer of more than 64 nodes or 60 layers ends the query unanswered.
+// Per query, layer by layer: the nodes whose control-point box (widened by max_edge) holds P run a
+// trajectory from their centre; a result counts when it converged inside the domain within max_edge
+// of P; the first layer with a result answers (its closest result; AMBIGUOUS as in the inversion);
+// otherwise each passing node is split by the reference's getSplitType and its children are the next
+// layer, in the reference's order.  The box checks and split decisions are exact (minima and maxima,
+// and getSplitType decided in FP32 only where its lengths are clearly off max_edge and else with the
+// reference-order FP64 functions; this translation unit is compiled with --fmad=false), so the tree
+// is the oracle's; the v-length uses the v-derivative, which the reference takes with
+// MatrixSurfaceDerivativeU.  With MODE mixed every node's trajectory runs in FP32 and its end takes
+// FP64 Newton steps (the mixed inversion's final steps).  Culled nodes are not split (their
+// control-point box does not hold P, so neither does their surface); a layer of more than 64 nodes or
+// 60 layers ends the query unanswered.
+//
+// Work distribution.  A persistent grid whose warps take portions of queries from a counter:
+//   1. root: the trajectories from the domain's centre stream through the warp's lanes (a lane whose
+//      query ended takes the portion's next one), their ends take the final FP64 steps 32 at a time.
+//      This answers most queries.
+//   2. the others collect in a queue; 32 at a time they are searched lane per query from the root's
+//      children on (the root's split does not depend on the query and is decided once per warp).
+//      Layers hold about one passing node, so a warp that searched one query at a time kept 1 lane
+//      in 32 busy.
+//   3. a query that meets a node of many control points, and the last one or two, are searched by the
+//      whole warp: lanes stride over a node's control points and take a node's trajectory each.
+// Measured on 2^18 points near the 64x64 surface (a search for 5 of every 32 queries), mixed: @@
 #include "invert_core.cuh"
 
 namespace gnurbs {
@@ -31,8 +36,13 @@ using namespace inv;
 
 constexpr int kQtMax = 64;     // nodes per layer (NODE_MAX_SIZE)
 constexpr int kQtLayers = 60;
+constexpr int kPortion = 128;   // queries a warp takes at a time, at most
+constexpr int kLaneCps = 512;   // control points of a node a lane scans alone
 
 struct QtWarp {
+  float ru[kPortion], rv[kPortion];   // mixed: ends of the root trajectories
+  unsigned char list[kPortion], end[kPortion];
+  long long rest[64];             // queries the root did not answer
   double node[2][kQtMax + 4][4];  // two layers: lb.u, lb.v, rt.u, rt.v
   int code[2][kQtMax + 4];        // index of the node's precomputed box, -1 when it has none
   double su[kQtMax], sv[kQtMax], sr[kQtMax];
@@ -76,8 +86,8 @@ __device__ int split_type(const SurfDev& s, const double* nd, double max_edge) {
 // and 256x256 nets, the FP32 lengths err by at most 1.4e-4 of themselves, so both give the same
 // decision; the FP32 one costs a fraction of the FP64 work (the FP64 split types took most of a
 // launch).
-template <int P, int Q>
-__device__ int split_type_fast(const SurfDev& s, const Ctx& cx, const double* nd, double max_edge) {
+template <class Eval>
+__device__ int split_type_fast(const SurfDev& s, const Eval& ev, const double* nd, double max_edge) {
   const double iu = (nd[2] - nd[0]) / 4, iv = (nd[3] - nd[1]) / 4;
   float ul = 0, vl = 0;
   bool exact = false;
@@ -85,8 +95,7 @@ __device__ int split_type_fast(const SurfDev& s, const Ctx& cx, const double* nd
     const double x = nd[0] + i * iu, y = nd[1] + i * iv;
     const int su = exact::find_seg(s.bu, s.ns_u, x), sv = exact::find_seg(s.bv, s.ns_v, y);
     int hu = su, hv = sv;
-    const fast::SDer<float> d = fast::eval_at<float, P, Q, 1, true>(cx.L32, cx.m32, cx.p, cx.q, (float)x, (float)y,
-                                                                  hu, hv);
+    const fast::SDer<float> d = ev.template at<1>((float)x, (float)y, hu, hv);
     exact = exact || hu != su || hv != sv;
     ul += sqrtf(dot3(d.Su, d.Su));
     vl += sqrtf(dot3(d.Sv, d.Sv));
@@ -111,38 +120,97 @@ __device__ __forceinline__ void put_node(double* o, double a, double b, double c
   o[3] = d;
 }
 
-// Precomputed boxes of the top kQtDepth levels of square children (depth d, u index a, v index b:
-// code = base(d) + a * 2^d + b; base = 0, 1, 5), written when the surface is converted.  Deeper
-// nodes, and the halves of U / V splits, scan their control points.
-constexpr int kQtDepth = 3;
-__device__ __forceinline__ int code_depth(int c) { return c == 0 ? 0 : (c < 5 ? 1 : 2); }
+// Precomputed boxes of the top kQuadtreeDepth levels of square children (depth d, u index a, v index
+// b: code = (4^d - 1) / 3 + a 2^d + b), written when the surface is converted.  Deeper nodes, and the
+// halves of U / V splits, scan their control points.
 __device__ __forceinline__ int child_code(int pc, int hu, int hv) {
   if (pc < 0) return -1;
-  const int d = code_depth(pc);
-  if (d + 1 >= kQtDepth) return -1;
-  const int base = d == 0 ? 0 : 1, side = 1 << d, idx = pc - base;
-  const int a = idx / side, b = idx % side;
-  return (d == 0 ? 1 : 5) + (2 * a + hu) * (2 * side) + (2 * b + hv);
+  int d = 0, base = 0;
+  while (pc >= base + (1 << (2 * d))) base += 1 << (2 * d++);
+  if (d + 1 >= kQuadtreeDepth) return -1;
+  const int a = (pc - base) >> d, b = (pc - base) & ((1 << d) - 1);
+  return base + (1 << (2 * d)) + ((2 * a + hu) << (d + 1)) + (2 * b + hv);
 }
 
 // Partial box over a node's control points (the rows findSpan(lb.u) - p .. findSpan(rt.u), the
-// same in v: BoundingBoxCheck's range), over elements t, t + stride, ...; starts from the first
-// control point of the range, as the reference does.
-__device__ void node_box(const SurfDev& s, const double* nd, int t, int stride, double* mn, double* mx) {
+// same in v: BoundingBoxCheck's range), over elements t, t + stride, ..., as order keys.
+struct CpRange {
+  int i0, j0, nb;
+  int64_t cnt;
+};
+__device__ __forceinline__ CpRange cp_range(const SurfDev& s, const double* nd) {
   const int i0 = knot_span(s.knot_u, s.bu, s.ns_u, nd[0]) - s.p, i1 = knot_span(s.knot_u, s.bu, s.ns_u, nd[2]);
   const int j0 = knot_span(s.knot_v, s.bv, s.ns_v, nd[1]) - s.q, j1 = knot_span(s.knot_v, s.bv, s.ns_v, nd[3]);
-  const int nb = j1 - j0 + 1, cnt = (i1 - i0 + 1) * nb;
+  const int nb = j1 - j0 + 1;
+  return {i0, j0, nb, (int64_t)(i1 - i0 + 1) * nb};
+}
+__device__ __forceinline__ void node_box(const SurfDev& s, const CpRange& r, int t, int stride, long long* mn,
+                                         long long* mx) {
   for (int c = 0; c < 3; ++c) {
-    mn[c] = s.cps[3 * ((size_t)i0 * s.nv + j0) + c];
-    mx[c] = mn[c];
+    mn[c] = 0x7fffffffffffffffll;
+    mx[c] = -0x7fffffffffffffffll - 1;
   }
-  for (int e = t; e < cnt; e += stride) {
-    const double* x = s.cps + 3 * ((size_t)(i0 + e / nb) * s.nv + (j0 + e % nb));
+  for (int64_t e = t; e < r.cnt; e += stride) {
+    const int row = (int)(e / r.nb), col = (int)(e - (int64_t)row * r.nb);
+    const double* x = s.cps + 3 * ((size_t)(r.i0 + row) * s.nv + (r.j0 + col));
     for (int c = 0; c < 3; ++c) {
-      mn[c] = mn[c] > x[c] ? x[c] : mn[c];
-      mx[c] = mx[c] < x[c] ? x[c] : mx[c];
+      const long long k = fast::order_key(x[c]);
+      mn[c] = k < mn[c] ? k : mn[c];
+      mx[c] = k > mx[c] ? k : mx[c];
     }
   }
+}
+__device__ __forceinline__ double key_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ bool box_holds(const double* mn, const double* mx, double px, double py, double pz,
+                                          double max_edge) {
+  return px >= mn[0] - max_edge && px <= mx[0] + max_edge && py >= mn[1] - max_edge && py <= mx[1] + max_edge &&
+         pz >= mn[2] - max_edge && pz <= mx[2] + max_edge;
+}
+// children of a node split by type t (1 V, 2 U, 3 both), in the reference's order; returns their number
+__device__ __forceinline__ int put_children(int type, const double* nd, int pc, double* o, int* oc) {
+  if (type == 0) return 0;
+  const double lx = nd[0], ly = nd[1], rx = nd[2], ry = nd[3];
+  const double mxu = (lx + rx) / 2, myv = (ly + ry) / 2;
+  if (type == 3) {
+    put_node(o, lx, ly, mxu, myv);
+    put_node(o + 4, lx, myv, mxu, ry);
+    put_node(o + 8, mxu, myv, rx, ry);
+    put_node(o + 12, mxu, ly, rx, myv);
+    oc[0] = child_code(pc, 0, 0);
+    oc[1] = child_code(pc, 0, 1);
+    oc[2] = child_code(pc, 1, 1);
+    oc[3] = child_code(pc, 1, 0);
+    return 4;
+  }
+  if (type == 2) {
+    put_node(o, lx, ly, mxu, ry);
+    put_node(o + 4, mxu, ly, rx, ry);
+  } else {
+    put_node(o, lx, ly, rx, myv);
+    put_node(o + 4, lx, myv, rx, ry);
+  }
+  oc[0] = oc[1] = -1;
+  return 2;
+}
+
+__device__ __forceinline__ void far_limits(const Ctx& c, float far[4]) {
+  const float eu = 2.0f * (float)(c.dom_u1 - c.dom_u0), ev = 2.0f * (float)(c.dom_v1 - c.dom_v0);
+  far[0] = (float)c.dom_u0 - eu;
+  far[1] = (float)c.dom_u1 + eu;
+  far[2] = (float)c.dom_v0 - ev;
+  far[3] = (float)c.dom_v1 + ev;
+}
+template <typename T>
+__device__ __forceinline__ void seed_start(T u, T v, Seed<T>& sd) {
+  sd.u = u;
+  sd.v = v;
+  sd.prev = INFINITY;
+  sd.it = 0;
+  sd.hu = 0;
+  sd.hv = 0;
+  sd.newton = false;
 }
 
 // One node's trajectory from (u, v): FP64 (the inversion's FP64 iteration), or MIXED (the mixed
@@ -150,39 +218,29 @@ __device__ void node_box(const SurfDev& s, const double* nd, int t, int stride, 
 // final steps).  True when it converged inside the domain within max_edge of P; (u, v, rr) the
 // result.
 template <int P, int Q, int MODE>
-__device__ bool node_trajectory(const SurfDev& s, const Ctx& cx, double px, double py, double pz, double max_edge,
-                                double& u, double& v, double& rr) {
+__device__ __noinline__ bool node_trajectory(const SurfDev& s, const SpanTables<kSmemSpans>& sm, double px, double py,
+                                             double pz, double max_edge, double& u, double& v, double& rr) {
+  const Ctx& cx = sm.ctx;
   if constexpr (MODE == kModeMixed) {
+    const StagedEval<P, Q, kSmemSpans> ev{sm};
     Seed<float> sd;
-    sd.u = (float)u;
-    sd.v = (float)v;
-    sd.prev = INFINITY;
-    sd.it = 0;
-    sd.hu = 0;
-    sd.hv = 0;
-    sd.newton = false;
+    seed_start((float)u, (float)v, sd);
     const float tx = (float)(px - s.org[0]), ty = (float)(py - s.org[1]), tz = (float)(pz - s.org[2]);
-    const float eu = 2.0f * (float)(s.dom_u1 - s.dom_u0), ev = 2.0f * (float)(s.dom_v1 - s.dom_v0);
-    const float far[4] = {(float)s.dom_u0 - eu, (float)s.dom_u1 + eu, (float)s.dom_v0 - ev, (float)s.dom_v1 + ev};
+    float far[4];
+    far_limits(cx, far);
     float dist;
     int r = kContinue;
     while (r == kContinue) {
-      r = iterate32(GlobalEval<P, Q>{cx}, tx, ty, tz, sd, dist);
+      r = iterate32(ev, tx, ty, tz, sd, dist);
       if (r == kContinue && !(sd.u >= far[0] && sd.u <= far[1] && sd.v >= far[2] && sd.v <= far[3])) r = kFailed;
     }
     if (r != kConverged) return false;
     u = sd.u;
     v = sd.v;
-    return final64<P, Q>(cx, px, py, pz, u, v, rr) && rr < max_edge;
+    return final64<P, Q>(cx, ev, px, py, pz, u, v, rr) && rr < max_edge;
   } else {
     Seed<double> sd;
-    sd.u = u;
-    sd.v = v;
-    sd.prev = INFINITY;
-    sd.it = 0;
-    sd.hu = 0;
-    sd.hv = 0;
-    sd.newton = false;
+    seed_start(u, v, sd);
     int r = kContinue;
     double dist2 = 0;
     while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd, dist2);
@@ -194,35 +252,101 @@ __device__ bool node_trajectory(const SurfDev& s, const Ctx& cx, double px, doub
   }
 }
 
-// The whole warp searches one query's tree.  root_failed: the root passed and its trajectory had
-// no result (the chunk's lane-per-query first layer found that), so layer 0 goes straight to the
-// split.
+// One lane searches one query's tree from the root's children on (the root passed and had no
+// result).  Returns the status, or -1 when the search meets a node of more than kLaneCps control
+// points (it is then the warp's).
 template <int P, int Q, int MODE>
-__device__ void quadtree_query(const SurfDev& s, const Ctx& cx, QtWarp& w, const double* __restrict__ qtbox,
-                               const double* __restrict__ Pq, int64_t qi, double max_edge, bool root_failed,
-                               double* __restrict__ uv_out, int* __restrict__ st_out, double* __restrict__ res_out) {
+__device__ __noinline__ int quadtree_lane(const SurfDev& s, const SpanTables<kSmemSpans>& sm, const double* __restrict__ qtbox,
+                             int root_type, double px, double py, double pz, double max_edge, double& ou, double& ov,
+                             double& orr) {
+  double node[2][kQtMax][4];
+  int code[2][kQtMax];
+  double ru[kQtMax], rv[kQtMax], rr[kQtMax];
+  const StagedEval<P, Q, kSmemSpans> ev{sm};
+  const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
+  int cur = 0, size = put_children(root_type, root, 0, node[0][0], code[0]);
+  for (int layer = 1; layer < kQtLayers && size > 0; ++layer) {
+    unsigned long long pass = 0;
+    for (int i = 0; i < size; ++i) {
+      const double* nd = node[cur][i];
+      double mn[3], mx[3];
+      if (code[cur][i] >= 0) {  // the top levels' boxes, written with the surface
+        const double* b = qtbox + 6 * code[cur][i];
+        for (int c = 0; c < 3; ++c) {
+          mn[c] = b[c];
+          mx[c] = b[3 + c];
+        }
+      } else {
+        const CpRange r = cp_range(s, nd);
+        if (r.cnt > kLaneCps) return -1;
+        long long kn[3], kx[3];
+        node_box(s, r, 0, 1, kn, kx);
+        for (int c = 0; c < 3; ++c) {
+          mn[c] = key_value(kn[c]);
+          mx[c] = key_value(kx[c]);
+        }
+      }
+      if (box_holds(mn, mx, px, py, pz, max_edge)) pass |= 1ull << i;
+    }
+    int nr = 0;
+    for (unsigned long long m = pass; m; m &= m - 1) {
+      const double* nd = node[cur][__ffsll((long long)m) - 1];
+      double u = (nd[0] + nd[2]) / 2, v = (nd[1] + nd[3]) / 2, r;
+      if (node_trajectory<P, Q, MODE>(s, sm, px, py, pz, max_edge, u, v, r)) {
+        ru[nr] = u;
+        rv[nr] = v;
+        rr[nr] = r;
+        ++nr;
+      }
+    }
+    if (nr > 0) {  // the layer's closest result (ties: the lower node)
+      int best = 0, status = 0;
+      for (int i = 1; i < nr; ++i)
+        if (rr[i] < rr[best]) best = i;
+      for (int i = 0; i < nr; ++i)
+        if (i != best && rr[i] <= rr[best] * (1 + 1e-6) + 1e-12 &&
+            (fabs(ru[i] - ru[best]) > 1e-7 || fabs(rv[i] - rv[best]) > 1e-7))
+          status = 1;
+      ou = ru[best];
+      ov = rv[best];
+      orr = rr[best];
+      return status;
+    }
+    int total = 0;
+    for (unsigned long long m = pass; m; m &= m - 1) {
+      const int i = __ffsll((long long)m) - 1;
+      const int type = split_type_fast(s, ev, node[cur][i], max_edge);
+      const int nch = type == 3 ? 4 : (type == 0 ? 0 : 2);
+      if (total + nch > kQtMax) return 3;  // layer overflow: unanswered
+      put_children(type, node[cur][i], code[cur][i], node[cur ^ 1][total], code[cur ^ 1] + total);
+      total += nch;
+    }
+    cur ^= 1;
+    size = total;
+  }
+  return 3;
+}
+
+// The whole warp searches one query's tree from the root's children on (the root passed and had no
+// result): a node's control-point box is reduced by the warp, the passing nodes' trajectories and
+// splits run one per lane.
+template <int P, int Q, int MODE>
+__device__ __noinline__ void quadtree_query(const SurfDev& s, const SpanTables<kSmemSpans>& sm, QtWarp& w,
+                               const double* __restrict__ qtbox, const double* __restrict__ Pq, int64_t qi,
+                               int root_type, double max_edge, double* __restrict__ uv_out, int* __restrict__ st_out, double* __restrict__ res_out) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const double px = Pq[3 * qi], py = Pq[3 * qi + 1], pz = Pq[3 * qi + 2];
-  int cur = 0, size = 1, status = 3;
-  bool passed_any = false;
+  const StagedEval<P, Q, kSmemSpans> ev{sm};
+  int cur = 0, status = 3;
+  const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
+  int size = root_type == 3 ? 4 : (root_type == 0 ? 0 : 2);
   double ou = __longlong_as_double(0x7ff8000000000000ll), ov = ou, orr = ou;
-  if (lane == 0) {
-    put_node(w.node[0][0], s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1);
-    w.code[0][0] = 0;
-  }
+  if (lane == 0) put_children(root_type, root, 0, w.node[0][0], w.code[0]);
   __syncwarp();
-  for (int layer = 0; layer < kQtLayers && size > 0; ++layer) {
-    const bool known = layer == 0 && root_failed;
-    if (known) {
-      if (lane == 0) {
-        w.pass[0] = 1;
-        w.ok[0] = 0;
-      }
-      passed_any = true;
-    }
+  for (int layer = 1; layer < kQtLayers && size > 0; ++layer) {
     // ---- control-point boxes (BoundingBoxCheck), one node at a time, the warp striding over it
-    for (int i = 0; i < (known ? 0 : size); ++i) {
+    for (int i = 0; i < size; ++i) {
       const double* nd = w.node[cur][i];
       double mn[3], mx[3];
       if (w.code[cur][i] >= 0) {  // the top levels' boxes, written with the surface
@@ -232,26 +356,29 @@ __device__ void quadtree_query(const SurfDev& s, const Ctx& cx, QtWarp& w, const
           mx[c] = b[3 + c];
         }
       } else {
-        node_box(s, nd, lane, 32, mn, mx);
+        long long kn[3], kx[3];
+        node_box(s, cp_range(s, nd), lane, 32, kn, kx);
         for (int o = 16; o > 0; o >>= 1)
           for (int c = 0; c < 3; ++c) {
-            mn[c] = fmin(mn[c], __shfl_xor_sync(FULL, mn[c], o));
-            mx[c] = fmax(mx[c], __shfl_xor_sync(FULL, mx[c], o));
+            const long long a = __shfl_xor_sync(FULL, kn[c], o), b = __shfl_xor_sync(FULL, kx[c], o);
+            kn[c] = a < kn[c] ? a : kn[c];
+            kx[c] = b > kx[c] ? b : kx[c];
           }
+        for (int c = 0; c < 3; ++c) {
+          mn[c] = key_value(kn[c]);
+          mx[c] = key_value(kx[c]);
+        }
       }
-      const bool pass = px >= mn[0] - max_edge && px <= mx[0] + max_edge && py >= mn[1] - max_edge &&
-                        py <= mx[1] + max_edge && pz >= mn[2] - max_edge && pz <= mx[2] + max_edge;
-      if (lane == 0) w.pass[i] = pass ? 1 : 0;
-      passed_any = passed_any || pass;
+      if (lane == 0) w.pass[i] = box_holds(mn, mx, px, py, pz, max_edge) ? 1 : 0;
     }
     __syncwarp();
     // ---- trajectories of the passing nodes, one per lane
-    for (int i = lane; i < (known ? 0 : size); i += 32) {
+    for (int i = lane; i < size; i += 32) {
       w.ok[i] = 0;
       if (!w.pass[i]) continue;
       const double* nd = w.node[cur][i];
       double u = (nd[0] + nd[2]) / 2, v = (nd[1] + nd[3]) / 2, rr;
-      if (node_trajectory<P, Q, MODE>(s, cx, px, py, pz, max_edge, u, v, rr)) {
+      if (node_trajectory<P, Q, MODE>(s, sm, px, py, pz, max_edge, u, v, rr)) {
         w.ok[i] = 1;
         w.su[i] = u;
         w.sv[i] = v;
@@ -279,7 +406,7 @@ __device__ void quadtree_query(const SurfDev& s, const Ctx& cx, QtWarp& w, const
     for (int r = 0; r < 2; ++r) {
       const int i = lane + 32 * r;
       if (i < size && w.pass[i]) {
-        typ[r] = split_type_fast<P, Q>(s, cx, w.node[cur][i], max_edge);
+        typ[r] = split_type_fast(s, ev, w.node[cur][i], max_edge);
         nch[r] = typ[r] == 3 ? 4 : (typ[r] == 0 ? 0 : 2);
       }
     }
@@ -294,36 +421,10 @@ __device__ void quadtree_query(const SurfDev& s, const Ctx& cx, QtWarp& w, const
       total += __shfl_sync(FULL, incl, 31);
     }
     if (total > kQtMax) break;  // layer overflow: unanswered
-    if (total == 0) {
-      status = passed_any ? 3 : 2;
-      break;
-    }
+    if (total == 0) break;
     for (int r = 0; r < 2; ++r) {
       const int i = lane + 32 * r;
-      if (nch[r] == 0) continue;
-      const double* nd = w.node[cur][i];
-      const double lx = nd[0], ly = nd[1], rx = nd[2], ry = nd[3];
-      const double mxu = (lx + rx) / 2, myv = (ly + ry) / 2;
-      double* o = w.node[cur ^ 1][off[r]];
-      int* oc = w.code[cur ^ 1] + off[r];
-      const int pc = w.code[cur][i];
-      if (typ[r] == 3) {
-        put_node(o, lx, ly, mxu, myv);
-        put_node(o + 4, lx, myv, mxu, ry);
-        put_node(o + 8, mxu, myv, rx, ry);
-        put_node(o + 12, mxu, ly, rx, myv);
-        const int hu[4] = {0, 0, 1, 1}, hv[4] = {0, 1, 1, 0};
-        for (int c = 0; c < 4; ++c) oc[c] = child_code(pc, hu[c], hv[c]);
-      } else {
-        if (typ[r] == 2) {
-          put_node(o, lx, ly, mxu, ry);
-          put_node(o + 4, mxu, ly, rx, ry);
-        } else {
-          put_node(o, lx, ly, rx, myv);
-          put_node(o + 4, lx, myv, rx, ry);
-        }
-        oc[0] = oc[1] = -1;
-      }
+      if (nch[r] > 0) put_children(typ[r], w.node[cur][i], w.code[cur][i], w.node[cur ^ 1][off[r]], w.code[cur ^ 1] + off[r]);
     }
     __syncwarp();
     cur ^= 1;
@@ -338,69 +439,172 @@ __device__ void quadtree_query(const SurfDev& s, const Ctx& cx, QtWarp& w, const
   __syncwarp();
 }
 
+// Register budget: 4 CTAs per SM (128 registers); the run-time degrees' variant 2.
 template <int P, int Q, int MODE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
     k_invert_quadtree(SurfDev s, const double* __restrict__ qtbox, const double* __restrict__ Pq, int64_t n,
                       double max_edge, double* __restrict__ uv_out, int* __restrict__ st_out,
-                      double* __restrict__ res_out, unsigned long long* __restrict__ counter) {
+                      double* __restrict__ res_out, unsigned long long* __restrict__ counter, float share,
+                      int least) {
+  __shared__ SpanTables<kSmemSpans> sm;
   __shared__ QtWarp ww[kWarps];
-  Ctx cx;
-  cx.L32 = fast::global_locator<float>(s);
-  cx.L64 = fast::global_locator<double>(s);
-  cx.m32 = s.m32;
-  cx.m64 = s.m64;
-  cx.p = s.p;
-  cx.q = s.q;
-  cx.dom_u0 = s.dom_u0;
-  cx.dom_u1 = s.dom_u1;
-  cx.dom_v0 = s.dom_v0;
-  cx.dom_v1 = s.dom_v1;
+  stage_tables(s, sm, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const Ctx& cx = sm.ctx;
+  const StagedEval<P, Q, kSmemSpans> ev{sm};
   QtWarp& w = ww[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const unsigned FULL = 0xffffffffu;
-  // chunks of 32 queries: the first layer (the root, one node) lane per query, which answers most
-  // queries; the warp then searches the rest one by one from the root's split
-  const int64_t chunks = (n + 31) / 32;
-  for (;;) {
-    unsigned long long ch = 0;
-    if (lane == 0) ch = atomicAdd(counter, 1ull);
-    ch = __shfl_sync(FULL, ch, 0);
-    if ((int64_t)ch >= chunks) break;
-    const int64_t qi = (int64_t)ch * 32 + lane;
-    bool rest = false;
-    if (qi < n) {
-      const double px = Pq[3 * qi], py = Pq[3 * qi + 1], pz = Pq[3 * qi + 2];
-      const bool pass = px >= qtbox[0] - max_edge && px <= qtbox[3] + max_edge && py >= qtbox[1] - max_edge &&
-                        py <= qtbox[4] + max_edge && pz >= qtbox[2] - max_edge && pz <= qtbox[5] + max_edge;
-      int status = 2;  // the root alone does not pass: no node ever passes
-      double ou = __longlong_as_double(0x7ff8000000000000ll), ov = ou, orr = ou;
-      if (pass) {
-        double u = (s.dom_u0 + s.dom_u1) / 2, v = (s.dom_v0 + s.dom_v1) / 2, rr = 0;
-        const bool ok = node_trajectory<P, Q, MODE>(s, cx, px, py, pz, max_edge, u, v, rr);
-        if (ok) {
-          status = 0;
-          ou = u;
-          ov = v;
-          orr = rr;
-        } else {
-          rest = true;
-        }
-      }
-      if (!rest) {
-        uv_out[2 * qi] = ou;
-        uv_out[2 * qi + 1] = ov;
-        st_out[qi] = status;
-        res_out[qi] = orr;
-      }
+  const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const double cu = (s.dom_u0 + s.dom_u1) / 2, cv = (s.dom_v0 + s.dom_v1) / 2;
+  float far[4];
+  far_limits(cx, far);
+  int nrest = 0, root_type = -1;
+  int64_t seen = 0;
+  auto answer = [&](int64_t q, int status, double u, double v, double r) {
+    uv_out[2 * q] = u;
+    uv_out[2 * q + 1] = v;
+    st_out[q] = status;
+    res_out[q] = r;
+  };
+  // the last `cnt` queries of the queue
+  auto search = [&](int cnt) {
+    if (root_type < 0) {
+      const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
+      root_type = split_type_fast(s, ev, root, max_edge);
     }
-    unsigned m = __ballot_sync(FULL, rest);
-    while (m) {
-      const int j = __ffs(m) - 1;
-      m &= m - 1;
-      quadtree_query<P, Q, MODE>(s, cx, w, qtbox, Pq, (int64_t)ch * 32 + j, max_edge, true, uv_out, st_out,
-                                 res_out);
+    nrest -= cnt;
+    unsigned byw = cnt <= 2 ? (1u << cnt) - 1u : 0u;  // searched by the whole warp
+    if (cnt > 2) {
+      bool big = false;
+      if (lane < cnt) {
+        const int64_t q = w.rest[nrest + lane];
+        double u = nan, v = nan, r = nan;
+        const int st = quadtree_lane<P, Q, MODE>(s, sm, qtbox, root_type, Pq[3 * q], Pq[3 * q + 1], Pq[3 * q + 2],
+                                                 max_edge, u, v, r);
+        big = st < 0;
+        if (!big) answer(q, st, u, v, r);
+      }
+      byw = __ballot_sync(FULL, big);
+    }
+    for (; byw; byw &= byw - 1)
+      quadtree_query<P, Q, MODE>(s, sm, w, qtbox, Pq, w.rest[nrest + __ffs(byw) - 1], root_type, max_edge, uv_out,
+                                 st_out, res_out);
+    __syncwarp();
+  };
+  // queues the queries of the lanes with `open`, and searches a full warp's worth
+  auto queue = [&](bool open, int64_t q) {
+    const unsigned m = __ballot_sync(FULL, open);
+    if (open) w.rest[nrest + __popc(m & lt_mask)] = q;
+    nrest += __popc(m);
+    __syncwarp();
+    if (nrest >= 32) search(32);
+  };
+  for (;;) {
+    // this warp's share of what is left, a few queries at least
+    const float fair = (float)(n - seen) * share;
+    const int want = max(fair < (float)kPortion ? (int)fair + 1 : kPortion, least);
+    unsigned long long a = 0;
+    if (lane == 0) a = atomicAdd(counter, (unsigned long long)want);
+    const int64_t q0 = (int64_t)__shfl_sync(FULL, a, 0);
+    if (q0 >= n) break;
+    seen = q0 + want;
+    const int cnt = (int)(n - q0 < want ? n - q0 : want);
+    // ---- the root's box: queries outside it have no candidate
+    int total = 0;
+    for (int base = 0; base < cnt; base += 32) {
+      const int k = base + lane;
+      bool pass = false;
+      if (k < cnt) {
+        const int64_t q = q0 + k;
+        pass = box_holds(qtbox, qtbox + 3, Pq[3 * q], Pq[3 * q + 1], Pq[3 * q + 2], max_edge);
+        if (!pass) answer(q, 2, nan, nan, nan);  // no node ever passes
+      }
+      const unsigned m = __ballot_sync(FULL, pass);
+      if (pass) w.list[total + __popc(m & lt_mask)] = (unsigned char)k;
+      total += __popc(m);
+    }
+    __syncwarp();
+    // ---- trajectories from the domain's centre
+    int next = 0, slot = 0;
+    bool waiting = true;
+    int end = kContinue;
+    typedef typename std::conditional<MODE == kModeMixed, float, double>::type T;
+    Seed<T> sd;
+    T tx = 0, ty = 0, tz = 0, dist = 0;
+    for (;;) {
+      const unsigned wm = __ballot_sync(FULL, waiting);
+      if (__popc(wm) >= (MODE == kModeMixed ? kStartBatch : kStartBatch64) || wm == FULL) {
+        if constexpr (MODE == kModeMixed) {
+          if (end != kContinue) {
+            w.end[slot] = (unsigned char)end;
+            w.ru[slot] = sd.u;
+            w.rv[slot] = sd.v;
+          }
+        } else {
+          bool open = false;
+          const int64_t q = q0 + w.list[slot];
+          if (end != kContinue) {
+            const double r = sqrt(dist);
+            if (end == kConverged && in_domain64(cx, sd.u, sd.v, dist) && r < max_edge) answer(q, 0, sd.u, sd.v, r);
+            else open = true;
+          }
+          queue(open, q);
+        }
+        end = kContinue;
+        if (next >= total && wm == FULL) break;
+        const int t = next + __popc(wm & lt_mask);
+        if (waiting && t < total) {
+          waiting = false;
+          slot = t;
+          const int64_t q = q0 + w.list[t];
+          if constexpr (MODE == kModeMixed) {
+            tx = (float)(Pq[3 * q] - s.org[0]);
+            ty = (float)(Pq[3 * q + 1] - s.org[1]);
+            tz = (float)(Pq[3 * q + 2] - s.org[2]);
+          } else {
+            tx = Pq[3 * q];
+            ty = Pq[3 * q + 1];
+            tz = Pq[3 * q + 2];
+          }
+          seed_start((T)cu, (T)cv, sd);
+        }
+        next = min(next + __popc(wm), total);
+      }
+      if (!waiting) {
+        if constexpr (MODE == kModeMixed) {
+          end = iterate32(ev, tx, ty, tz, sd, dist);
+          if (end == kContinue && !(sd.u >= far[0] && sd.u <= far[1] && sd.v >= far[2] && sd.v <= far[3])) end = kFailed;
+        } else {
+          end = iterate64<P, Q>(cx, tx, ty, tz, sd, dist);
+        }
+        waiting = end != kContinue;
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+    // ---- MIXED: the final FP64 steps of their ends
+    if constexpr (MODE == kModeMixed) {
+      for (int base = 0; base < total; base += 32) {
+        const int k = base + lane;
+        bool open = false;
+        int64_t q = 0;
+        if (k < total) {
+          q = q0 + w.list[k];
+          open = true;
+          if (w.end[k] == kConverged) {
+            double u = w.ru[k], v = w.rv[k], r;
+            if (final64<P, Q>(cx, ev, Pq[3 * q], Pq[3 * q + 1], Pq[3 * q + 2], u, v, r) && r < max_edge) {
+              answer(q, 0, u, v, r);
+              open = false;
+            }
+          }
+        }
+        queue(open, q);
+      }
     }
   }
+  if (nrest > 0) search(nrest);
 }
 
 template <int P, int Q, int MODE>
@@ -417,10 +621,14 @@ cudaError_t launch_quadtree_mode(const SurfDev& s, const double* P_, int64_t n, 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_invert_quadtree<P, Q, MODE>, kThreads, 0);
     cached[dev] = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   }
-  int64_t blocks = ((n + 31) / 32 + kWarps - 1) / kWarps;
+  // as many warps as take at least one query per scheduler of the launch (up to 32: a pass of the
+  // final steps costs as much for one), at most the resident ones
+  const int64_t spread = n / kSchedulers;
+  const int least = (int)(spread < 1 ? 1 : (spread < 32 ? spread : 32));
+  int64_t blocks = ((n + least - 1) / least + kWarps - 1) / kWarps;
   if (blocks > cached[dev]) blocks = cached[dev];
   k_invert_quadtree<P, Q, MODE><<<(unsigned)blocks, kThreads, 0, st>>>(s, s.qtbox, P_, n, max_edge, uv, st_, res,
-                                                                       counter);
+                                                                       counter, 1.0f / (float)(blocks * kWarps), least);
   return cudaGetLastError();
 }
 

@@ -81,16 +81,17 @@ __device__ __forceinline__ double warp_pick(double x) {
 }
 __device__ __forceinline__ double shfl(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
 
-// Control points acting on the parameter rectangle lb..rt: order keys of their minima (0..2) and
-// maxima (3..5) over the CTA's threads.
-__device__ __forceinline__ void hull_of(const SurfDev& s, int a0, int a1, int b0, int b1, long long h[6]) {
+// Control points a0..a1 x b0..b1: order keys of their minima (0..2) and maxima (3..5) over the
+// elements t, t + stride, ..., reduced over the warp.
+__device__ __forceinline__ void hull_of(const SurfDev& s, int a0, int a1, int b0, int b1, int t, int stride,
+                                        long long h[6]) {
   const int nb = b1 - b0 + 1;
   const int64_t cnt = (int64_t)(a1 - a0 + 1) * nb;
   for (int c = 0; c < 3; ++c) {
     h[c] = 0x7fffffffffffffffll;
     h[3 + c] = -0x7fffffffffffffffll - 1;
   }
-  for (int64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
+  for (int64_t e = t; e < cnt; e += stride) {
     const int row = (int)(e / nb), col = (int)(e - (int64_t)row * nb);
     const double* x = s.cps + 3 * ((size_t)(a0 + row) * s.nv + (b0 + col));
 #pragma unroll
@@ -279,7 +280,8 @@ __device__ __forceinline__ void node_samples(const SurfDev& s, int k) {
     if (i1 > i0 && s.bu[i1] >= ur) --i1;  // the span starting at the right end
     if (j1 > j0 && s.bv[j1] >= vr) --j1;
     long long hull[6];
-    hull_of(s, s.knot_u[i0] - p, s.knot_u[i1], s.knot_v[j0] - q, s.knot_v[j1], hull);
+    hull_of(s, s.knot_u[i0] - p, s.knot_u[i1], s.knot_v[j0] - q, s.knot_v[j1], threadIdx.x, blockDim.x,
+            hull);
     if (lane < 3) {
       red[warp].nmax[c] = hi;
       red[warp].nmin[c] = lo;
@@ -442,12 +444,14 @@ __device__ __forceinline__ void node_finish(const SurfDev& s, int k) {
   for (int c = 15; c < kConeStride; ++c) rec[c] = 0;
 }
 
-// Control-point box of one of the quadtree inversion's precomputed nodes: the top levels of square
-// children (depth d, u index a, v index b: code = base(d) + a * 2^d + b; base = 0, 1, 5), the node's
-// rectangle by the search's own midpoint splits, the control points of BoundingBoxCheck's range.
-__device__ __forceinline__ void quadtree_box(const SurfDev& s, int code) {
-  const int d = code == 0 ? 0 : (code < 5 ? 1 : 2), side = 1 << d, idx = code - (d == 0 ? 0 : (d == 1 ? 1 : 5));
-  const int a = idx / side, b = idx % side;
+// Control-point box of one of the quadtree inversion's precomputed nodes (kQuadtreeDepth levels of
+// square children: depth d, u index a, v index b, code = (4^d - 1) / 3 + a 2^d + b), the node's
+// rectangle by the search's own midpoint splits, the control points of BoundingBoxCheck's range: the
+// part of threads t, t + stride, ..., reduced over the warp.
+__device__ __forceinline__ void quadtree_box(const SurfDev& s, int code, int t, int stride, long long h[6]) {
+  int d = 0, base = 0;
+  while (code >= base + (1 << (2 * d))) base += 1 << (2 * d++);
+  const int a = (code - base) >> d, b = (code - base) & ((1 << d) - 1);
   double nd[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
   for (int l = d - 1; l >= 0; --l) {
     const double mu = (nd[0] + nd[2]) / 2, mv = (nd[1] + nd[3]) / 2;
@@ -455,9 +459,14 @@ __device__ __forceinline__ void quadtree_box(const SurfDev& s, int code) {
     if ((b >> l) & 1) nd[1] = mv; else nd[3] = mv;
   }
   auto knot = [](const int* idx_of, const double* br, int ns, double x) { return idx_of[exact::find_seg(br, ns, x)]; };
-  long long h[6];
   hull_of(s, knot(s.knot_u, s.bu, s.ns_u, nd[0]) - s.p, knot(s.knot_u, s.bu, s.ns_u, nd[2]),
-          knot(s.knot_v, s.bv, s.ns_v, nd[1]) - s.q, knot(s.knot_v, s.bv, s.ns_v, nd[3]), h);
+          knot(s.knot_v, s.bv, s.ns_v, nd[1]) - s.q, knot(s.knot_v, s.bv, s.ns_v, nd[3]), t, stride, h);
+}
+
+constexpr int kQuadtreeLarge = 1 + 4 + 16;  // boxes of depth 0..2: a CTA each; the deeper ones a warp each
+__device__ __forceinline__ void quadtree_box_cta(const SurfDev& s, int code) {
+  long long h[6];
+  quadtree_box(s, code, threadIdx.x, blockDim.x, h);
   __shared__ long long red[kNodeWarps][6];
   if ((threadIdx.x & 31) == 0)
     for (int c = 0; c < 6; ++c) red[threadIdx.x >> 5][c] = h[c];
@@ -469,12 +478,19 @@ __device__ __forceinline__ void quadtree_box(const SurfDev& s, int code) {
     s.qtbox[6 * code + c] = key_value(k);
   }
 }
-
-constexpr int kQuadtreeBoxes = 1 + 4 + 16;
+__device__ __forceinline__ void quadtree_box_warp(const SurfDev& s, int code) {
+  if (code >= kQuadtreeBoxes) return;
+  long long h[6];
+  quadtree_box(s, code, threadIdx.x & 31, 32, h);
+  if ((threadIdx.x & 31) == 0)
+    for (int c = 0; c < 6; ++c) s.qtbox[6 * code + c] = key_value(h[c]);
+}
 
 __global__ void __launch_bounds__(kNodeThreads) k_nodes(SurfDev s) {
-  if (blockIdx.x < kTreeNodes) node_samples<true>(s, blockIdx.x);
-  else quadtree_box(s, blockIdx.x - kTreeNodes);
+  const int b = blockIdx.x;
+  if (b < kTreeNodes) node_samples<true>(s, b);
+  else if (b < kTreeNodes + kQuadtreeLarge) quadtree_box_cta(s, b - kTreeNodes);
+  else quadtree_box_warp(s, kQuadtreeLarge + (b - kTreeNodes - kQuadtreeLarge) * kNodeWarps + (threadIdx.x >> 5));
 }
 __global__ void __launch_bounds__(32) k_nodes_finish(SurfDev s) { node_finish<true>(s, blockIdx.x); }
 
@@ -517,7 +533,8 @@ __global__ void k_candidates(SurfDev s, const double* __restrict__ P, int64_t n,
 }
 
 cudaError_t launch_nodes(const SurfDev& s, cudaStream_t st) {
-  k_nodes<<<kTreeNodes + kQuadtreeBoxes, kNodeThreads, 0, st>>>(s);
+  constexpr int small = (kQuadtreeBoxes - kQuadtreeLarge + kNodeWarps - 1) / kNodeWarps;
+  k_nodes<<<kTreeNodes + kQuadtreeLarge + small, kNodeThreads, 0, st>>>(s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_nodes_finish<<<kTreeNodes, 32, 0, st>>>(s);

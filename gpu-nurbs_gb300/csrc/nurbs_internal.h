@@ -21,6 +21,8 @@ inline int64_t span_blocks(int q, int64_t nspans) { return (nspans + span_group(
 constexpr int kGap = 8;           // GapPerEdge (src/kernel/kernel.cuh:17)
 constexpr int kPts = kGap + 1;    // PointsPerEdge
 constexpr int kConeStride = 20;   // floats per normal-cone record
+constexpr int kQuadtreeDepth = 5;  // levels of the quadtree inversion with precomputed boxes
+constexpr int kQuadtreeBoxes = ((1 << (2 * kQuadtreeDepth)) - 1) / 3;  // 341
 
 // Device view of one surface.  All pointers are device pointers into the surface's arena.
 //
@@ -47,8 +49,9 @@ constexpr int kConeStride = 20;   // floats per normal-cone record
 //                                    rt 12..14), zero (15..19)
 //   lattice[65][81][3]               surface points of each node's 9x9 lattice (index 9 tx + ty),
 //                                    FP32 relative to org: distance bounds and projection seeds
-//   qtbox[21][6]                     control-point boxes of the quadtree inversion's square nodes of
-//                                    depth 0..2, written with the tree
+//   qtbox[341][6]                    control-point boxes of the quadtree inversion's square nodes of
+//                                    depth 0..4, written with the tree
+// (pooled surfaces, which are only inverted and evaluated, have no nbox, cone, lattice and qtbox)
 struct SurfDev {
   int p, q, nu, nv;
   int ns_u, ns_v;
@@ -84,7 +87,7 @@ struct SurfDev {
   double* nbox;           // normal cones (see above)
   float* cone;
   float* lattice;
-  double* qtbox;          // control-point boxes of the quadtree inversion's top levels (21 x 6)
+  double* qtbox;          // control-point boxes of the quadtree inversion's top levels
 };
 
 // Tree node in the reference TreeNode order (src/kernel/kernel.cuh:30-39), 80 bytes.

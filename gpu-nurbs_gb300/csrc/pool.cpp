@@ -336,7 +336,7 @@ int nurbs_pool_add(nurbs_pool_t P, int count, const nurbs_surface_desc* descs, v
   size_t in_total = 0;
   for (int k = 0; k < count; ++k) {
     const nurbs_surface_desc& d = descs[k];
-    int rc = prepare_surface(d.degree_u, d.degree_v, d.cp_u, d.cp_v, d.knots_u, d.knots_v, d.cps, d.weights, S[k], err);
+    int rc = prepare_surface(d.degree_u, d.degree_v, d.cp_u, d.cp_v, d.knots_u, d.knots_v, d.cps, d.weights, S[k], err, false);
     if (rc) return pfail(rc, "surface %d: %s", k, err.c_str());
     in_total += S[k].in_bytes;
   }
@@ -466,7 +466,7 @@ int nurbs_pool_surface_bytes(int p, int q, int nu, int nv, const double* ku, con
   std::vector<double> cps((size_t)nu * nv * 3, 0.0), w((size_t)nu * nv, 1.0);
   SurfaceHost S;
   std::string err;
-  int rc = prepare_surface(p, q, nu, nv, ku, kv, cps.data(), w.data(), S, err);
+  int rc = prepare_surface(p, q, nu, nv, ku, kv, cps.data(), w.data(), S, err, false);
   if (rc) return pfail(rc, "%s", err.c_str());
   *bytes = (int64_t)(align256(S.in_bytes) + align256(S.out_bytes));
   return NURBS_OK;

@@ -35,6 +35,7 @@ inline void breakpoints(const double* k, int p, int cp, std::vector<double>& b, 
 // matrices and basis matrices, written by the conversion kernels).
 struct SurfaceHost {
   int p = 0, q = 0, nu = 0, nv = 0;
+  bool culling = false;
   std::vector<double> ku, kv, bu, bv, idu, idv, cps, w;
   std::vector<float> bu32, bv32, idu32, idv32;
   std::vector<int> iu, iv;
@@ -46,9 +47,9 @@ struct SurfaceHost {
 };
 
 // Validates and prepares a surface given by host arrays.  Returns NURBS_OK or an error code,
-// with a message in err.
+// with a message in err.  culling: with room for the projection's and the quadtree inversion's data.
 inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const double* kv, const double* cps,
-                           const double* w, SurfaceHost& S, std::string& err) {
+                           const double* w, SurfaceHost& S, std::string& err, bool culling) {
   auto bad = [&](int code, const std::string& m) {
     err = m;
     return code;
@@ -115,10 +116,13 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
   S.o_bas_v = take((size_t)nsv * (q + 1) * (q + 1) * 8);
   S.o_cd32 = take((kTreeNodes * 9 + 1) * 4);
   S.o_cd64 = take(kTreeNodes * 9 * 8);
-  S.o_nbox = take(kTreeNodes * 6 * 8);
-  S.o_cone = take(kTreeNodes * kConeStride * 4);
-  S.o_lat = take(kTreeNodes * kPts * kPts * 3 * 4);
-  S.o_qtb = take(21 * 6 * 8);
+  S.culling = culling;
+  if (culling) {
+    S.o_nbox = take(kTreeNodes * 6 * 8);
+    S.o_cone = take(kTreeNodes * kConeStride * 4);
+    S.o_lat = take(kTreeNodes * kPts * kPts * 3 * 4);
+    S.o_qtb = take(kQuadtreeBoxes * 6 * 8);
+  }
   S.out_bytes = off;
   return NURBS_OK;
 }
@@ -175,10 +179,12 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.basis_v = (double*)(out_dev + S.o_bas_v);
   d.cd32 = (float*)(out_dev + S.o_cd32);
   d.cd64 = (double*)(out_dev + S.o_cd64);
-  d.nbox = (double*)(out_dev + S.o_nbox);
-  d.cone = (float*)(out_dev + S.o_cone);
-  d.lattice = (float*)(out_dev + S.o_lat);
-  d.qtbox = (double*)(out_dev + S.o_qtb);
+  if (S.culling) {
+    d.nbox = (double*)(out_dev + S.o_nbox);
+    d.cone = (float*)(out_dev + S.o_cone);
+    d.lattice = (float*)(out_dev + S.o_lat);
+    d.qtbox = (double*)(out_dev + S.o_qtb);
+  }
 }
 
 }  // namespace gnurbs
