@@ -418,6 +418,7 @@ __device__ __forceinline__ int finish_status(const double* us, const double* vs,
 // most KS spans per direction.
 template <int KS>
 struct SpanTables {
+  static_assert(kGridBuckets % KS == 0, "the staged grid is a thinned one");
   Ctx ctx;    // one copy for all threads, its fields read where they are used
   bool fits;  // breakpoint tables staged
   // FP32 breakpoints and inverse span lengths, and a lookup grid over the domain: KS equal buckets,
@@ -453,13 +454,12 @@ __device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& s
       const float *b = dir ? s.bv32 : s.bu32, *inv = dir ? s.inv_dv32 : s.inv_du32;
       const int ns = dir ? s.ns_v : s.ns_u;
       for (int k = tid; k <= ns; k += nthreads) sm.seg[dir][k] = make_float2(b[k], k < ns ? inv[k] : 0.f);
-      // a bucket's points are right of this value whatever the rounding of their bucket index
-      const float g0 = b[0], gs = (float)KS / (b[ns] - b[0]);
-      for (int i = tid; i < KS; i += nthreads)
-        sm.grid[dir][i] = i == 0 ? 0 : (unsigned char)fast::find_seg(b, ns, g0 + ((float)i - 0.01f) / gs);
+      // the surface's lookup grid, thinned to KS buckets
+      const unsigned char* grid = dir ? s.grid_v : s.grid_u;
+      for (int i = tid; i < KS; i += nthreads) sm.grid[dir][i] = grid[i * (kGridBuckets / KS)];
       if (tid == 0) {
-        sm.g0[dir] = g0;
-        sm.gs[dir] = gs;
+        sm.g0[dir] = dir ? s.g0_v : s.g0_u;
+        sm.gs[dir] = (dir ? s.gs_v : s.gs_u) * ((float)KS / kGridBuckets);
       }
     }
   }

@@ -7,6 +7,7 @@ namespace gnurbs {
 
 constexpr int kMaxDegree = 7;     // p, q <= 7 (reference MAX_DEGREE 8 = p+1)
 constexpr int kTreeNodes = 65;    // root + 8x8 children
+constexpr int kGridBuckets = 256;  // of a direction's span lookup grid
 
 // Coefficients per span in the FP32 span table: (p+1)(q+1) rounded up to even, so every span
 // starts 32-byte aligned and coefficient pairs can be read with one 256-bit load.
@@ -30,6 +31,8 @@ constexpr int kQuadtreeBoxes = ((1 << (2 * kQuadtreeDepth)) - 1) / 3;  // 341
 //   bu[ns_u+1], bv[ns_v+1]           breakpoints = distinct knots of the domain, ascending
 //   inv_du[ns_u], inv_dv[ns_v]       1/(bu[s+1]-bu[s])
 //   bu32/bv32, inv_du32/inv_dv32     the same in FP32 (mixed-precision seeding)
+//   grid_u[256], grid_v[256]         FP32 span lookup: per bucket of 1/256 of the domain the span of its
+//                                    left end (or one before), for directions of at most 256 spans
 //   knot_u[ns_u], knot_v[ns_v]       knot index m of span s (k[m] = bu[s]) for the reference layout
 //   m64[ns_u*ns_v][k1][k2][4]        span matrices, homogeneous components (xw, yw, zw, w)
 //                                    innermost, so one (a,b) coefficient is one 32-byte vector
@@ -68,6 +71,9 @@ struct SurfDev {
   const float* bv32;
   const float* inv_du32;
   const float* inv_dv32;
+  const unsigned char* grid_u;  // lookup grids (see above); null with more than kGridBuckets spans
+  const unsigned char* grid_v;
+  float g0_u, gs_u, g0_v, gs_v;  // bucket of x: (x - g0) * gs
   const int* knot_u;
   const int* knot_v;
   const double* m64;

@@ -30,6 +30,22 @@ inline void breakpoints(const double* k, int p, int cp, std::vector<double>& b, 
   }
 }
 
+// Lookup grid of the FP32 breakpoints b: per bucket i of (x - b[0]) * kGridBuckets / extent, a span no
+// later than that of any of its points (the bucket's left end moved left by a hundredth of a bucket,
+// far more than the rounding of a bucket index).
+inline void span_grid(const std::vector<float>& b, std::vector<unsigned char>& grid) {
+  const int ns = (int)b.size() - 1;
+  grid.clear();
+  if (ns > kGridBuckets) return;
+  grid.resize(kGridBuckets);
+  const double step = ((double)b[ns] - b[0]) / kGridBuckets;
+  for (int i = 0, k = 0; i < kGridBuckets; ++i) {
+    const double x = b[0] + (i - 0.01) * step;
+    while (k < ns - 1 && b[k + 1] <= x) ++k;
+    grid[i] = (unsigned char)k;
+  }
+}
+
 // Everything the device block of one surface is built from.  Its block has two parts: the
 // input part (uploaded: tables, knots, control net, zeroed tree) and the computed part (span
 // matrices and basis matrices, written by the conversion kernels).
@@ -39,8 +55,9 @@ struct SurfaceHost {
   std::vector<double> ku, kv, bu, bv, idu, idv, cps, w;
   std::vector<float> bu32, bv32, idu32, idv32;
   std::vector<int> iu, iv;
+  std::vector<unsigned char> gu, gv;  // span lookup grids (empty with more than kGridBuckets spans)
   // offsets inside the input part
-  size_t o_bu, o_bv, o_idu, o_idv, o_bu32, o_bv32, o_idu32, o_idv32, o_iu, o_iv, o_ku, o_kv, o_cps, o_w, o_tree,
+  size_t o_bu, o_bv, o_idu, o_idv, o_bu32, o_bv32, o_idu32, o_idv32, o_iu, o_iv, o_gu, o_gv, o_ku, o_kv, o_cps, o_w, o_tree,
       o_div, o_built, in_bytes;
   // offsets inside the computed part
   size_t o_m64, o_m32, o_bas_u, o_bas_v, o_cd32, o_cd64, o_nbox, o_cone, o_lat, o_qtb, out_bytes;
@@ -92,6 +109,8 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
   S.bv32.assign(S.bv.begin(), S.bv.end());
   for (int i = 0; i < nsu; ++i) S.idu[i] = 1.0 / (S.bu[i + 1] - S.bu[i]), S.idu32[i] = (float)S.idu[i];
   for (int i = 0; i < nsv; ++i) S.idv[i] = 1.0 / (S.bv[i + 1] - S.bv[i]), S.idv32[i] = (float)S.idv[i];
+  span_grid(S.bu32, S.gu);
+  span_grid(S.bv32, S.gv);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -103,6 +122,7 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
   S.o_bu32 = take((nsu + 1) * 4); S.o_bv32 = take((nsv + 1) * 4);
   S.o_idu32 = take(nsu * 4); S.o_idv32 = take(nsv * 4);
   S.o_iu = take(nsu * 4); S.o_iv = take(nsv * 4);
+  S.o_gu = take(kGridBuckets); S.o_gv = take(kGridBuckets);
   S.o_ku = take(S.ku.size() * 8); S.o_kv = take(S.kv.size() * 8);
   S.o_cps = take(ncp * 3 * 8); S.o_w = take(ncp * 8);
   S.o_tree = take(kTreeNodes * sizeof(TreeNodeDev));
@@ -144,6 +164,8 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   put(S.o_idv32, S.idv32.data(), nsv * 4);
   put(S.o_iu, S.iu.data(), nsu * 4);
   put(S.o_iv, S.iv.data(), nsv * 4);
+  put(S.o_gu, S.gu.data(), S.gu.size());
+  put(S.o_gv, S.gv.data(), S.gv.size());
   put(S.o_ku, S.ku.data(), S.ku.size() * 8);
   put(S.o_kv, S.kv.data(), S.kv.size() * 8);
   put(S.o_cps, S.cps.data(), S.cps.size() * 8);
@@ -168,6 +190,12 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.inv_du = (const double*)(in_dev + S.o_idu); d.inv_dv = (const double*)(in_dev + S.o_idv);
   d.bu32 = (const float*)(in_dev + S.o_bu32); d.bv32 = (const float*)(in_dev + S.o_bv32);
   d.inv_du32 = (const float*)(in_dev + S.o_idu32); d.inv_dv32 = (const float*)(in_dev + S.o_idv32);
+  d.grid_u = S.gu.empty() ? nullptr : (const unsigned char*)(in_dev + S.o_gu);
+  d.grid_v = S.gv.empty() ? nullptr : (const unsigned char*)(in_dev + S.o_gv);
+  d.g0_u = S.bu32[0];
+  d.gs_u = (float)kGridBuckets / (S.bu32[nsu] - S.bu32[0]);
+  d.g0_v = S.bv32[0];
+  d.gs_v = (float)kGridBuckets / (S.bv32[nsv] - S.bv32[0]);
   d.knot_u = (const int*)(in_dev + S.o_iu); d.knot_v = (const int*)(in_dev + S.o_iv);
   d.knots_u = (const double*)(in_dev + S.o_ku); d.knots_v = (const double*)(in_dev + S.o_kv);
   d.cps = (const double*)(in_dev + S.o_cps); d.weights = (const double*)(in_dev + S.o_w);
