@@ -385,6 +385,30 @@ struct Horner {
   }
 };
 
+// Horner<double, D> of one component.
+template <int D>
+struct HornerOne {
+  double p, dp, ddp;
+  int k;
+  GN_HD HornerOne() : p(0), dp(0), ddp(0), k(0) {}
+  GN_HD void push(double c, double x) {
+    if (k == 0) {
+      p = c;
+    } else {
+      if (D >= 2) {
+        if (k == 2) ddp = dp;
+        else if (k > 2) ddp = mad(ddp, x, dp);
+      }
+      if (D >= 1) {
+        if (k == 1) dp = p;
+        else dp = mad(dp, x, p);
+      }
+      p = mad(p, x, c);
+    }
+    ++k;
+  }
+};
+
 template <typename T>
 GN_HD v4<T> zero4() {
   return {T(0), T(0), T(0), T(0)};
