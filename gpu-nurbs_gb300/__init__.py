@@ -195,16 +195,26 @@ def write_nu(path: str, surf: dict):
 
 
 # -------------------------------------------------------------------------- helpers
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream(stream=None):
+    """The given stream, or the handle of torch's current one (read without making a Stream object,
+    which costs a small call more than its launch)."""
     if stream is not None:
         return stream
     torch = _torch()
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _ptr(t) -> int:

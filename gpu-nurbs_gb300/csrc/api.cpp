@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -107,12 +108,8 @@ int validate_knots(const double* k, int p, int cp, const char* name) {
 }
 
 // Host copy of a buffer given as host or device pointer.
-int fetch(const double* src, size_t n, int kind, std::vector<double>& dst, cudaStream_t st) {
+int fetch(const double* src, size_t n, std::vector<double>& dst, cudaStream_t st) {
   dst.resize(n);
-  if (kind == NURBS_PTR_HOST) {
-    std::memcpy(dst.data(), src, n * sizeof(double));
-    return NURBS_OK;
-  }
   CUDA_TRY(cudaMemcpyAsync(dst.data(), src, n * sizeof(double), cudaMemcpyDeviceToHost, st), "copy to host");
   CUDA_TRY(cudaStreamSynchronize(st), "stream sync");
   return NURBS_OK;
@@ -179,7 +176,6 @@ static cudaError_t invert_on(nurbs_surface_s* s, const double* P, int64_t n, dou
 static void release_surface(nurbs_surface_s* s) {
   for (cudaEvent_t& ev : s->done)
     if (ev) cudaEventDestroy(ev);
-  if (s->counters) cudaFree(s->counters);
 }
 
 extern "C" {
@@ -225,18 +221,25 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
   // device inputs are read back once: validation and breakpoint tables are host work
   std::vector<double> ku, kv, hc, hw;
   const size_t ncp = (size_t)nu * nv;
-  if ((rc = fetch(knots_u, p + nu + 1, ptr_kind, ku, st))) return rc;
-  if ((rc = fetch(knots_v, q + nv + 1, ptr_kind, kv, st))) return rc;
-  if ((rc = fetch(cps, ncp * 3, ptr_kind, hc, st))) return rc;
-  if ((rc = fetch(weights, ncp, ptr_kind, hw, st))) return rc;
+  if (ptr_kind != NURBS_PTR_HOST) {
+    if ((rc = fetch(knots_u, p + nu + 1, ku, st))) return rc;
+    if ((rc = fetch(knots_v, q + nv + 1, kv, st))) return rc;
+    if ((rc = fetch(cps, ncp * 3, hc, st))) return rc;
+    if ((rc = fetch(weights, ncp, hw, st))) return rc;
+    knots_u = ku.data();
+    knots_v = kv.data();
+    cps = hc.data();
+    weights = hw.data();
+  }
   SurfaceHost S;
   std::string err;
-  if ((rc = prepare_surface(p, q, nu, nv, ku.data(), kv.data(), hc.data(), hw.data(), S, err, true)))
+  if ((rc = prepare_surface(p, q, nu, nv, knots_u, knots_v, cps, weights, S, err, true)))
     return fail(rc, "%s", err.c_str());
   nurbs_surface_s* s = new (std::nothrow) nurbs_surface_s();
   if (!s) return fail(NURBS_E_NOMEM, "host allocation failed");
   cudaGetDevice(&s->device);
-  const size_t total = S.in_bytes + S.out_bytes;
+  // one allocation: the input part, the computed part, the launch counters
+  const size_t total = S.in_bytes + S.out_bytes + align256(sizeof(unsigned long long) * kCounterRing);
   cudaError_t e = cudaMalloc(&s->arena, total);
   if (e != cudaSuccess) {
     delete s;
@@ -265,13 +268,7 @@ int nurbs_surface_create(int p, int q, int nu, int nv, const double* knots_u, co
     return cuda_fail(e, "matrix-form conversion");
   }
   s->tree_built = true;
-  e = cudaMalloc((void**)&s->counters, sizeof(unsigned long long) * kCounterRing);
-  if (e != cudaSuccess) {
-    cudaFree(s->arena);
-    delete s;
-    cudaGetLastError();
-    return fail(NURBS_E_NOMEM, "device allocation of the launch counters failed: %s", cudaGetErrorString(e));
-  }
+  s->counters = (unsigned long long*)(A + S.in_bytes + S.out_bytes);
   *out = s;
   return NURBS_OK;
 }
@@ -313,8 +310,8 @@ int nurbs_get_matrix_n_raw(double* matrix_n_dev, int p, int q, int nu, int nv, c
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   std::vector<double> ku, kv;
-  if ((rc = fetch(knots_u_dev, p + nu + 1, NURBS_PTR_DEVICE, ku, st))) return rc;
-  if ((rc = fetch(knots_v_dev, q + nv + 1, NURBS_PTR_DEVICE, kv, st))) return rc;
+  if ((rc = fetch(knots_u_dev, p + nu + 1, ku, st))) return rc;
+  if ((rc = fetch(knots_v_dev, q + nv + 1, kv, st))) return rc;
   if ((rc = validate_knots(ku.data(), p, nu, "knots_u"))) return rc;
   if ((rc = validate_knots(kv.data(), q, nv, "knots_v"))) return rc;
   std::vector<double> bu, bv;
@@ -415,20 +412,33 @@ int nurbs_build_tree(nurbs_surface_t s, int levels, void* stream) {
 int nurbs_tree_export(nurbs_surface_t s, double* nodes_host, unsigned char* divided_host, unsigned char* built_host) {
   if (!s || !nodes_host || !divided_host || !built_host) return fail(NURBS_E_INVALID, "NULL argument");
   static_assert(sizeof(TreeNodeDev) == 80, "TreeNodeDev layout");
-  CUDA_TRY(cudaMemcpy(nodes_host, s->dev.tree, kTreeNodes * sizeof(TreeNodeDev), cudaMemcpyDeviceToHost), "tree copy");
-  CUDA_TRY(cudaMemcpy(divided_host, s->dev.divided, kTreeNodes, cudaMemcpyDeviceToHost), "divided copy");
-  CUDA_TRY(cudaMemcpy(built_host, s->dev.built, kTreeNodes, cudaMemcpyDeviceToHost), "built copy");
+  // the three are neighbours in the arena: one copy
+  const unsigned char* first = (const unsigned char*)s->dev.tree;
+  const size_t o_div = s->dev.divided - first, o_built = s->dev.built - first;
+  const size_t bytes = o_built + kTreeNodes;
+  std::unique_ptr<unsigned char[]> buf(new (std::nothrow) unsigned char[bytes]);
+  if (!buf) return fail(NURBS_E_NOMEM, "host allocation failed");
+  CUDA_TRY(cudaMemcpy(buf.get(), first, bytes, cudaMemcpyDeviceToHost), "tree copy");
+  std::memcpy(nodes_host, buf.get(), kTreeNodes * sizeof(TreeNodeDev));
+  std::memcpy(divided_host, buf.get() + o_div, kTreeNodes);
+  std::memcpy(built_host, buf.get() + o_built, kTreeNodes);
   return NURBS_OK;
 }
 
 int nurbs_normal_cones_export(nurbs_surface_t s, double* nbox_host, float* cone_host, float* lattice_host) {
   if (!s || !nbox_host || !cone_host || !lattice_host) return fail(NURBS_E_INVALID, "NULL argument");
-  CUDA_TRY(cudaMemcpy(nbox_host, s->dev.nbox, kTreeNodes * 6 * sizeof(double), cudaMemcpyDeviceToHost), "cone copy");
-  CUDA_TRY(cudaMemcpy(cone_host, s->dev.cone, kTreeNodes * kConeStride * sizeof(float), cudaMemcpyDeviceToHost),
-           "cone copy");
-  CUDA_TRY(cudaMemcpy(lattice_host, s->dev.lattice, kTreeNodes * kPts * kPts * 3 * sizeof(float),
-                      cudaMemcpyDeviceToHost),
-           "lattice copy");
+  // the three are neighbours in the arena: one copy
+  const size_t b_nbox = kTreeNodes * 6 * sizeof(double), b_cone = kTreeNodes * kConeStride * sizeof(float),
+               b_lat = kTreeNodes * kPts * kPts * 3 * sizeof(float);
+  const char* first = (const char*)s->dev.nbox;
+  const size_t o_cone = (const char*)s->dev.cone - first, o_lat = (const char*)s->dev.lattice - first;
+  const size_t bytes = o_lat + b_lat;
+  std::unique_ptr<char[]> buf(new (std::nothrow) char[bytes]);
+  if (!buf) return fail(NURBS_E_NOMEM, "host allocation failed");
+  CUDA_TRY(cudaMemcpy(buf.get(), first, bytes, cudaMemcpyDeviceToHost), "cone copy");
+  std::memcpy(nbox_host, buf.get(), b_nbox);
+  std::memcpy(cone_host, buf.get() + o_cone, b_cone);
+  std::memcpy(lattice_host, buf.get() + o_lat, b_lat);
   return NURBS_OK;
 }
 

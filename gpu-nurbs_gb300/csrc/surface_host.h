@@ -52,7 +52,8 @@ inline void span_grid(const std::vector<float>& b, std::vector<unsigned char>& g
 struct SurfaceHost {
   int p = 0, q = 0, nu = 0, nv = 0;
   bool culling = false;
-  std::vector<double> ku, kv, bu, bv, idu, idv, cps, w;
+  std::vector<double> ku, kv, bu, bv, idu, idv;
+  const double *cps = nullptr, *w = nullptr;  // the caller's control net: it outlives this
   std::vector<float> bu32, bv32, idu32, idv32;
   std::vector<int> iu, iv;
   std::vector<unsigned char> gu, gv;  // span lookup grids (empty with more than kGridBuckets spans)
@@ -96,8 +97,8 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
   S.p = p; S.q = q; S.nu = nu; S.nv = nv;
   S.ku.assign(ku, ku + p + nu + 1);
   S.kv.assign(kv, kv + q + nv + 1);
-  S.cps.assign(cps, cps + 3 * ncp);
-  S.w.assign(w, w + ncp);
+  S.cps = cps;
+  S.w = w;
   breakpoints(S.ku.data(), p, nu, S.bu, S.iu);
   breakpoints(S.kv.data(), q, nv, S.bv, S.iv);
   const int nsu = (int)S.iu.size(), nsv = (int)S.iv.size();
@@ -168,8 +169,9 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   put(S.o_gv, S.gv.data(), S.gv.size());
   put(S.o_ku, S.ku.data(), S.ku.size() * 8);
   put(S.o_kv, S.kv.data(), S.kv.size() * 8);
-  put(S.o_cps, S.cps.data(), S.cps.size() * 8);
-  put(S.o_w, S.w.data(), S.w.size() * 8);
+  const size_t ncp = (size_t)S.nu * S.nv;
+  put(S.o_cps, S.cps, ncp * 3 * 8);
+  put(S.o_w, S.w, ncp * 8);
   d = SurfDev{};
   d.p = S.p; d.q = S.q; d.nu = S.nu; d.nv = S.nv; d.ns_u = nsu; d.ns_v = nsv;
   d.range_u = S.ku[S.p + S.nu] - S.ku[0];  // kernel.cu:167
@@ -179,7 +181,7 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.dom_u0 = S.ku[S.p]; d.dom_u1 = S.ku[S.nu]; d.dom_v0 = S.kv[S.q]; d.dom_v1 = S.kv[S.nv];
   for (int c = 0; c < 3; ++c) {
     double lo = S.cps[c], hi = S.cps[c];
-    for (size_t k = 3 + c; k < S.cps.size(); k += 3) {
+    for (size_t k = 3 + c; k < 3 * ncp; k += 3) {
       lo = std::min(lo, S.cps[k]);
       hi = std::max(hi, S.cps[k]);
     }
