@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -30,14 +31,21 @@ inline void breakpoints(const double* k, int p, int cp, std::vector<double>& b, 
   }
 }
 
-// Lookup grid of the FP32 breakpoints b: per bucket i of (x - b[0]) * kGridBuckets / extent, a span no
-// later than that of any of its points (the bucket's left end moved left by a hundredth of a bucket,
-// far more than the rounding of a bucket index).
+// Lookup grid of the FP32 breakpoints b: bucket (x - b[0]) * grid_scale(b).  A zero, subnormal or
+// infinite FP32 extent has the scale 0: every point is then in bucket 0, span 0, and the search goes on
+// from there.
+inline float grid_scale(const std::vector<float>& b) {
+  const float g = (float)kGridBuckets / (b.back() - b[0]);
+  return g <= std::numeric_limits<float>::max() ? g : 0.f;
+}
+// Per bucket a span no later than that of any of its points (the bucket's left end moved left by a
+// hundredth of a bucket, far more than the rounding of a bucket index).
 inline void span_grid(const std::vector<float>& b, std::vector<unsigned char>& grid) {
   const int ns = (int)b.size() - 1;
   grid.clear();
   if (ns > kGridBuckets) return;
   grid.resize(kGridBuckets);
+  if (grid_scale(b) == 0.f) return;
   const double step = ((double)b[ns] - b[0]) / kGridBuckets;
   for (int i = 0, k = 0; i < kGridBuckets; ++i) {
     const double x = b[0] + (i - 0.01) * step;
@@ -195,9 +203,9 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.grid_u = S.gu.empty() ? nullptr : (const unsigned char*)(in_dev + S.o_gu);
   d.grid_v = S.gv.empty() ? nullptr : (const unsigned char*)(in_dev + S.o_gv);
   d.g0_u = S.bu32[0];
-  d.gs_u = (float)kGridBuckets / (S.bu32[nsu] - S.bu32[0]);
+  d.gs_u = grid_scale(S.bu32);
   d.g0_v = S.bv32[0];
-  d.gs_v = (float)kGridBuckets / (S.bv32[nsv] - S.bv32[0]);
+  d.gs_v = grid_scale(S.bv32);
   d.knot_u = (const int*)(in_dev + S.o_iu); d.knot_v = (const int*)(in_dev + S.o_iv);
   d.knots_u = (const double*)(in_dev + S.o_ku); d.knots_v = (const double*)(in_dev + S.o_kv);
   d.cps = (const double*)(in_dev + S.o_cps); d.weights = (const double*)(in_dev + S.o_w);
