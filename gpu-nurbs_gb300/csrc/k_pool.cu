@@ -1,37 +1,21 @@
 // Batched inversion over a pool of many surfaces of uneven degree, net size and query count,
 // in one persistent launch.
 //
-// The batch is cut on the host into tiles (surface, query range), listed surface by surface; a
-// group of consecutive tiles of one surface is one run of queries.  Large tiles go to CTAs: the
-// surface is staged once for four warps, which take equal portions of the run from a cursor in
-// shared memory.  Tiles of at most 32 queries (latency) go to warps, each staging the surface in its
-// own shared-memory area; warps never wait for one another, so a batch of a few thousand queries
-// spreads over all SMs.  Either way the queries stream through the warp's slots as in the
-// single-surface kernel (invert_core.cuh).  Degree dispatch: (p,q) in {2,3,5}^2 run
-// degree-specialised code, other degrees a run-time-degree path.  Tile size and CTAs per SM
-// are chosen by the pool's autotuner.
+// The batch is cut on the host into tiles (surface, query range), listed surface by surface.  A CTA
+// takes a tile, or a few consecutive small ones, from a counter; consecutive tiles of one surface are
+// one run of queries.  The surface of a run is staged once for the CTA's four warps, which take equal
+// portions of the run from a cursor in shared memory and stream them through their slots as in the
+// single-surface kernel (invert_core.cuh).  Degree dispatch: (p,q) in {2,3,5}^2 run degree-specialised
+// code, other degrees a run-time-degree path.  Tile size and CTAs per SM are chosen by the pool's
+// autotuner.
+#include <algorithm>
+
 #include "invert_core.cuh"
 
 namespace gnurbs {
 namespace {
 
 using namespace inv;
-
-// Each degree variant is its own (not inlined) function, so that it keeps its own register
-// allocation instead of the kernel taking the union of all variants' live ranges.
-constexpr int kPoolSpans = 64;  // breakpoint tables staged per warp up to this many spans
-
-// The queries [q, qend), handed to one warp.
-struct WarpRange {
-  int64_t q, qend;
-  __device__ __forceinline__ int grab(int want, int64_t& q0) {
-    q0 = q;
-    const int64_t left = qend - q;
-    const int k = left < want ? (int)left : want;
-    q += k;
-    return k;
-  }
-};
 
 // The queries from `begin` to `qend`, handed out to the CTA's warps by a cursor in shared memory,
 // `portion` at a time.
@@ -49,6 +33,8 @@ struct CtaRange {
   }
 };
 
+// Each degree variant is its own (not inlined) function, so that it keeps its own register
+// allocation instead of the kernel taking the union of all variants' live ranges.
 template <int P, int Q, int MODE, int KS, class Source>
 __device__ __noinline__ void stream_variant(Staged<KS, MODE>& sm, WarpWork<MODE>& ww,
                                             const double* __restrict__ P_, Source& src, double* __restrict__ uv,
@@ -90,41 +76,6 @@ __device__ __forceinline__ int tile_run(const InvTile* __restrict__ tiles, int t
   return t;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kThreads, 4) k_invert_pool(const SurfDev* __restrict__ table,
-                                                          const InvTile* __restrict__ tiles, int ntiles,
-                                                          int* __restrict__ counter, const double* __restrict__ P,
-                                                          double* __restrict__ uv, int* __restrict__ st,
-                                                          double* __restrict__ res, int group) {
-  __shared__ Staged<kPoolSpans, MODE> sm[kWarps];
-  __shared__ WarpWork<MODE> ww[kWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int cur = -1;
-  for (;;) {
-    // a group of consecutive chunks (mostly of one surface: chunks are listed surface by
-    // surface) per grab, so a warp restages rarely
-    int t0 = 0;
-    if (lane == 0) t0 = atomicAdd(counter, group);
-    t0 = __shfl_sync(0xffffffffu, t0, 0);
-    if (t0 >= ntiles) break;
-    const int t1 = min(t0 + group, ntiles);
-    for (int t = t0; t < t1;) {
-      int surf;
-      int64_t begin, end;
-      t = tile_run(tiles, t, t1, surf, begin, end);
-      if (surf != cur) {
-        __syncwarp();
-        const SurfDev s = table[surf];
-        stage_surface<kPoolSpans>(s, sm[warp], lane, 32);
-        cur = surf;
-        __syncwarp();
-      }
-      dispatch_stream<MODE>(sm[warp], ww[warp], P, WarpRange{begin, end}, uv, st, res);
-      __syncwarp();
-    }
-  }
-}
-
 // Batched FP64 evaluation over tiles: one CTA per tile, one thread per (u,v), run-time degrees.
 template <int ORDER>
 __global__ void __launch_bounds__(128) k_eval_pool(const SurfDev* __restrict__ table, const InvTile* __restrict__ tiles,
@@ -157,14 +108,17 @@ __global__ void __launch_bounds__(128) k_eval_pool(const SurfDev* __restrict__ t
   }
 }
 
-// CTA-granular schedule for large batches: a CTA takes a group of consecutive tiles, stages the
-// surface of each run of tiles once for its four warps, and the warps share the run's queries.
-constexpr int kCtaSpans = 256;
+constexpr int kCtaSpans = 256;      // breakpoint tables staged up to this many spans
+constexpr int kGroupQueries = 128;  // small tiles are taken together up to this many queries
+constexpr int kCtasPerSm = 4;
 
 // Register budget: 4 CTAs per SM (6 / 5 / 4: 6.95 / 6.32 / 6.01 ms on 160 uneven faces in tiles of 128;
-// every tile ends with its warps waiting for the last one, so latency counts).
+// every tile ends with its warps waiting for the last one, so latency counts).  Small tiles (32 queries
+// at most, for latency) are CTA work too: with a warp per tile, a batch's warps ran up to nine degree
+// variants side by side, each with a staged surface and a drain of its own.  Mixed, tiles of 16:
+// 1,000 queries of 3 surfaces 538 -> 221 us, 14,000 of 25 565 -> 450, 63,000 of 130 2348 -> 1317.
 template <int MODE>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
     k_invert_pool_cta(const SurfDev* __restrict__ table, const InvTile* __restrict__ tiles, int ntiles,
                       int* __restrict__ counter, const double* __restrict__ P, double* __restrict__ uv,
                       int* __restrict__ st, double* __restrict__ res, int group) {
@@ -217,30 +171,18 @@ cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int n
   if (ntiles <= 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
-  if (tile_queries > 32) {  // CTA tiles
-    if (ctas > ntiles) ctas = ntiles;
-    int group = ntiles / (ctas * 8);
-    group = group < 1 ? 1 : (group > 8 ? 8 : group);
-    if (precision == 1)
-      k_invert_pool_cta<kModeMixed><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
-                                                                group);
-    else
-      k_invert_pool_cta<kModeFP64><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
-                                                               group);
-    return cudaGetLastError();
-  }
-  const int warps_needed = ntiles;
-  if (ctas * kWarps > warps_needed) ctas = (warps_needed + kWarps - 1) / kWarps;
-  // chunks per grab: large batches take up to 8 at a time, while every warp still gets about
-  // eight grabs so the tail stays short
-  int group = ntiles / (ctas * kWarps * 8);
-  group = group < 1 ? 1 : (group > 8 ? 8 : group);
+  if (ctas > ntiles) ctas = ntiles;
+  // Tiles per grab: small tiles together, up to kGroupQueries queries, while every resident CTA gets a
+  // grab.  Larger tiles one by one: groups of 8 / 2 / 1 tiles of 128 take 41.3 / 35.8 / 32.8 ms on 600
+  // surfaces with 4.4 M queries (the last groups are the launch's tail), and the same on 300 with 1 M.
+  const int resident = std::min(ctas, kCtasPerSm * 152);
+  const int group = std::max(1, std::min(ntiles / resident, kGroupQueries / tile_queries));
   if (precision == 1)
-    k_invert_pool<kModeMixed><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
-                                                          group);
+    k_invert_pool_cta<kModeMixed><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
+                                                             group);
   else
-    k_invert_pool<kModeFP64><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
-                                                         group);
+    k_invert_pool_cta<kModeFP64><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
+                                                            group);
   return cudaGetLastError();
 }
 

@@ -474,7 +474,7 @@ int nurbs_pool_surface_bytes(int p, int q, int nu, int nv, const double* ku, con
 
 int nurbs_pool_set_config(nurbs_pool_t P, int tile_queries, int ctas_per_sm) {
   if (!P || tile_queries < 1 || (tile_queries > 32 && tile_queries % 32) || ctas_per_sm < 1 || ctas_per_sm > 16)
-    return pfail(NURBS_E_INVALID, "tile_queries must be 1..32 (warp chunks) or a multiple of 32 (CTA tiles), "
+    return pfail(NURBS_E_INVALID, "tile_queries must be 1..32 (latency) or a multiple of 32 (throughput), "
                                   "ctas_per_sm in 1..16");
   std::lock_guard<std::mutex> lock(P->mu);
   P->tile_queries = tile_queries;
@@ -548,7 +548,7 @@ int nurbs_pool_autotune(nurbs_pool_t P, int nbatch, const int* ids, const int64_
         return NURBS_OK;
       }
   }
-  // above 32: CTA tiles (throughput); 32 and below: warp chunks (latency, small batches)
+  // above 32: throughput; 32 and below: latency, small batches
   const int tile_opts[] = {128, 256, 32, 16};
   const int cta_opts[] = {4, 5, 6};
   cudaEvent_t e0, e1;

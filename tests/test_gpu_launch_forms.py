@@ -130,3 +130,25 @@ def test_search_of_part_of_a_launch(nurbs, pq, which, precision):
             found = t <= 1
             assert np.all(np.abs(u - uv[at])[found] <= 1e-9), (n, step)
             assert np.all(np.abs(r - res[at])[found] <= 1e-12 * res[at][found] + 1e-14), (n, step)
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_pool_tiles_taken_together(nurbs, precision):
+    """Small tiles are taken several at a time, across surfaces too: the single surfaces' bits for every tile
+    size, with more tiles than resident CTAs, empty and ragged ranges and a repeated surface."""
+    surfs = [surface(p, q, 9, 8, 20 + p + q) for p, q in ((3, 3), (2, 5), (4, 3), (5, 5))]
+    counts = [0, 1, 700, 17, 0, 33, 1300, 128]
+    which = [0, 1, 2, 3, 1, 0, 0, 2]
+    pool = nurbs.Pool(1 << 26, max_surfaces=8)
+    ids = pool.add(surfs)
+    singles = [nurbs.Surface(x) for x in surfs]
+    P = np.concatenate([queries(singles[w], nurbs, max(c, 1), 30 + k, 1e-2)[:c]
+                        for k, (w, c) in enumerate(zip(which, counts))])
+    off = np.concatenate([[0], np.cumsum(counts)])
+    batch = nurbs.Batch(np.asarray(ids)[which], off)
+    ref = [np.concatenate(x) for x in zip(*(host(*singles[w].invert(T(P[a:b]), precision))
+                                            for w, a, b in zip(which, off[:-1], off[1:]) if b > a))]
+    for tile in (1, 2, 16, 31, 32, 64, 256):
+        pool.set_config(tile, 6)
+        for a, b in zip(host(*pool.invert(batch, T(P), precision)), ref):
+            assert np.array_equal(a, b, equal_nan=True), tile
