@@ -117,7 +117,7 @@ int fetch(const double* src, size_t n, std::vector<double>& dst, cudaStream_t st
 
 }  // namespace
 
-// Inversion launches take their chunk counter from a ring of device words.  A slot is reused
+// Inversion launches take their query counter from a ring of device words.  A slot is reused
 // only after the launch that used it before has finished on the GPU (an event per slot), so
 // calls on several streams at once never share a counter.
 constexpr int kCounterRing = 16;

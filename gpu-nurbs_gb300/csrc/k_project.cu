@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, (MODE == kModeMixed && P != 0) ? 4 :
 template <int P, int Q, int MODE>
 cudaError_t launch_project_mode(const SurfDev& s, const double* P_, int64_t n, double* uv, int* st_, double* res,
                                 unsigned long long* counter, cudaStream_t st) {
-  if ((n + 31) / 32 > 0x3fffffffLL) return cudaErrorInvalidValue;  // chunk ids are 32-bit
+  if ((n + 31) / 32 > 0x3fffffffLL) return cudaErrorInvalidValue;  // far beyond any device's memory
   constexpr size_t bytes = ProjSmem<MODE>::bytes;
   static int cached[64] = {0};
   int dev = 0;

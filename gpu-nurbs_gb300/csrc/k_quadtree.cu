@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
 template <int P, int Q, int MODE>
 cudaError_t launch_quadtree_mode(const SurfDev& s, const double* P_, int64_t n, double max_edge, double* uv, int* st_,
                                  double* res, unsigned long long* counter, cudaStream_t st) {
-  if ((n + 31) / 32 > 0xffffffffLL) return cudaErrorInvalidValue;  // chunk ids are 32-bit
+  if ((n + 31) / 32 > 0xffffffffLL) return cudaErrorInvalidValue;  // far beyond any device's memory
   static int cached[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);

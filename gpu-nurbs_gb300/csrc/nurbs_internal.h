@@ -159,7 +159,7 @@ cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int n
                                const double* P, double* uv, int* status, double* residual, int precision,
                                int ctas, int tile_queries, cudaStream_t st);
 
-// stage d.  counter: one device word, zero when the launch starts (the kernel's chunk counter).
+// stage d.  counter: one device word, zero when the launch starts (queries handed out).
 cudaError_t launch_invert(const SurfDev& s, const double* P, int64_t n, double* uv, int* status,
                           double* residual, int precision, unsigned long long* counter, cudaStream_t st);
 // p-curves: continuation from the neighbours' pass-1 answers, then flags (k_pcurve.cu)
