@@ -9,9 +9,8 @@
 //
 // Two launches.  k_nodes: one CTA per node evaluates the node's samples and reduces them to the
 // unclipped box, the unclipped normal box and the control-point box; a node's samples do not
-// depend on its parent, so both levels run at once (the seed centres' derivatives and the quadtree
-// boxes are further CTAs of the same launch).  k_nodes_finish: a warp per node clips to the root
-// and writes the records.
+// depend on its parent, so both levels run at once (the quadtree boxes are further CTAs of the same
+// launch).  k_nodes_finish: a warp per node clips to the root and writes the records.
 //
 // What bounds it: FP64 arithmetic in the reference's order.  An FP64 instruction of a warp takes 64
 // clocks here whatever its active lanes, so the build is a question of how few of them follow one
