@@ -105,7 +105,33 @@ struct Ctx {
   const double* m64;
   int p, q;
   double dom_u0, dom_u1, dom_v0, dom_v1;
+  bool unit_range;   // both knot ranges are 1
+  double iru, irv;   // 1 / knot range, set when they are not
 };
+__device__ __forceinline__ void set_range(const SurfDev& s, Ctx& c) {
+  const long long one = __double_as_longlong(1.0);
+  c.unit_range = __double_as_longlong(s.range_u) == one && __double_as_longlong(s.range_v) == one;
+  c.iru = c.irv = 1.0;
+  if (!c.unit_range) {
+    c.iru = 1.0 / s.range_u;
+    c.irv = 1.0 / s.range_v;
+  }
+}
+
+// |S - P|^2 at (u - du, v - dv) from r = S - P, Su, Sv at (u, v): S(u - du, v - dv) = S - Su du -
+// Sv dv + O(|S''| 1e-20) for the steps a seed ends with (1e-10 at most), below the rounding of S
+// itself.  Su and Sv are scaled by the knot range (kernel.cu:167), so the steps are divided by it.
+__device__ __forceinline__ double dist2_after(const Ctx& c, const v3<double>& r, const v3<double>& Su,
+                                              const v3<double>& Sv, double du, double dv) {
+  if (!c.unit_range) {
+    du *= c.iru;
+    dv *= c.irv;
+  }
+  const v3<double> r2 = {fast::mad(-Sv.x, dv, fast::mad(-Su.x, du, r.x)),
+                         fast::mad(-Sv.y, dv, fast::mad(-Su.y, du, r.y)),
+                         fast::mad(-Sv.z, dv, fast::mad(-Su.z, du, r.z))};
+  return dot3(r2, r2);
+}
 
 // The FP32 evaluation of S..Svv that the explorations iterate with, from a context's tables
 // (GlobalEval: breakpoints by bisection from the last span) or from a staged surface (StagedEval).
@@ -163,9 +189,8 @@ __device__ __forceinline__ int iterate32(const Eval& ev, float px, float py, flo
 }
 
 // One FP64 iteration of a seed (FP64 mode).  dist2, when the seed converges: |S - P|^2 at the new
-// (u, v) from this step's S, Su, Sv: S(u - du, v - dv) = S - Su du - Sv dv + O(|S''| 1e-20), below
-// the rounding of S itself (another evaluation for the few lanes whose seeds just ended would cost
-// the warp as much as one for all lanes).
+// (u, v) from this step's S, Su, Sv (another evaluation for the few lanes whose seeds just ended would
+// cost the warp as much as one for all lanes).
 template <int P, int Q>
 __device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, double pz, Seed<double>& st,
                                          double& dist2) {
@@ -178,10 +203,7 @@ __device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, dou
   st.v -= dv;
   const double step = fast::max_abs(du, dv);
   if ((st.newton && fast::le_nonneg(step, kTolNewton64)) || fast::le_nonneg(step, kTolAny64)) {
-    const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
-                           fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
-                           fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-    dist2 = dot3(r2, r2);
+    dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   st.prev = step;
@@ -280,12 +302,7 @@ __device__ __forceinline__ int final_step(const Ctx& c, const Eval& ev, double p
   f.u -= du;
   f.v -= dv;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
-    // Residual at the returned point from this step's FP64 S, Su, Sv: S(u - du, v - dv) =
-    // S - Su du - Sv dv + O(|S''| 1e-20), below the rounding of S itself.
-    const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
-                           fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
-                           fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-    const double dist2 = dot3(r2, r2);
+    const double dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
     res = sqrt(dist2);
     return in_domain64(c, f.u, f.v, dist2) ? kConverged : kFailed;
   }
@@ -473,6 +490,7 @@ __device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& s
     cx.p = s.p;
     cx.q = s.q;
     cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
+    set_range(s, cx);
   }
 }
 

@@ -94,8 +94,8 @@ struct PSeed {
 // accepted point twice and hold up the warp for its longest search.  dist2: the squared distance, FP32
 // before the last step, FP64 at the end point.
 template <typename T>
-__device__ __forceinline__ int project_advance(const fast::SDer<T>& d, const T dom[4], T px, T py, T pz, PSeed<T>& st,
-                                               T& dist2) {
+__device__ __forceinline__ int project_advance(const Ctx& c, const fast::SDer<T>& d, const T dom[4], T px, T py, T pz,
+                                               PSeed<T>& st, T& dist2) {
   constexpr bool kFp32 = sizeof(T) == 4;
   const v3<T> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   const T fn = dot3(r, r);
@@ -175,12 +175,7 @@ __device__ __forceinline__ int project_advance(const fast::SDer<T>& d, const T d
   st.trial = false;
   const T du = st.u - st.un, dv = st.v - st.vn;
   if (moved_to()) {
-    if constexpr (!kFp32) {  // S(u - du, v - dv) = S - Su du - Sv dv, the rest below its rounding
-      const v3<T> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
-                        fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
-                        fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-      dist2 = dot3(r2, r2);
-    }
+    if constexpr (!kFp32) dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   return ++st.it >= kMaxIterProj ? kFailed : kContinue;
@@ -235,7 +230,7 @@ __device__ __forceinline__ int project_by_warp(const Eval& ev, const T dom[4], i
       st.vn = __shfl_sync(FULL, tv, first);
       st.ls = kMaxHalvings;  // taken
     }
-    const int res = project_advance(ev.template at<2>(st.un, st.vn, hu, hv), dom, px, py, pz, st, dist2);
+    const int res = project_advance(ev.sm.ctx, ev.template at<2>(st.un, st.vn, hu, hv), dom, px, py, pz, st, dist2);
     if (res != kContinue) return res;
   }
 }
@@ -285,10 +280,7 @@ __device__ __forceinline__ int project_polish_step(const Ctx& c, const Eval& ev,
   f.u = un;
   f.v = vn;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewtonProj)) {
-    const v3<double> r2 = {fast::mad(-d.Sv.x, dv, fast::mad(-d.Su.x, du, r.x)),
-                           fast::mad(-d.Sv.y, dv, fast::mad(-d.Su.y, du, r.y)),
-                           fast::mad(-d.Sv.z, dv, fast::mad(-d.Su.z, du, r.z))};
-    const double dist2 = dot3(r2, r2);
+    const double dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
     res = sqrt(dist2);
     return fast::is_finite(dist2) ? kConverged : kFailed;
   }
@@ -615,7 +607,7 @@ __device__ __forceinline__ void project_stream(const Staged<kSmemSpans, MODE>& s
         }
       }
       if (!waiting) {
-        const int res = project_advance(ev.template at<2>(sd.un, sd.vn, hu, hv), dom, tx, ty, tz, sd, dist);
+        const int res = project_advance(cx, ev.template at<2>(sd.un, sd.vn, hu, hv), dom, tx, ty, tz, sd, dist);
         if (res != kContinue) {
           end = res;
           waiting = true;
