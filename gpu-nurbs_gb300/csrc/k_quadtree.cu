@@ -20,14 +20,20 @@
 //   1. root: the trajectories from the domain's centre stream through the warp's lanes (a lane whose
 //      query ended takes the portion's next one), their ends take the final FP64 steps 32 at a time.
 //      This answers most queries.
-//   2. the others collect in a queue; 32 at a time they are searched lane per query from the root's
-//      children on (the root's split does not depend on the query and is decided once per warp).
-//      Layers hold about one passing node, so a warp that searched one query at a time kept 1 lane
-//      in 32 busy.
-//   3. a query that meets a node of many control points, and the last one or two, are searched by the
-//      whole warp: lanes stride over a node's control points and take a node's trajectory each.
-// Measured on 2^18 points near the 64x64 surface (a search for 5 of every 32 queries), mixed:
-// 3.2 ms with the warp per query, 1.7 ms so.
+//   2. the others collect in a queue; 32 at a time they are searched layer by layer from the root's
+//      children on, a query per lane (the root's split does not depend on the query and is decided once
+//      per warp).  Layers hold about one passing node, so a warp that searched one query at a time kept
+//      1 lane in 32 busy.  The trajectories and splits of the layer's passing nodes are one list of
+//      tasks for all lanes, and a node of many control points is scanned by the whole warp, so neither
+//      makes one lane the last.
+//   3. a query whose layer outgrows what a lane keeps is searched on by the whole warp, a node per lane.
+// Measured with a warp per query / a lane per query, its trajectories one after the other / now:
+//   64x64 surface, mixed, 2^18 points within 5e-5      2,585 / 1,557 / 1,181 us  (max_edge 1e-4)
+//   64x64 surface, mixed, 20,000 points off by ~3e-5   1,339 / 3,204 /   729 us  (max_edge 1e-4)
+//   8x8 rough surface, FP64, 20,000 off by ~3e-2       5,172 / 52,467 / 4,103 us (max_edge 0.1: wide layers)
+//   degrees 7 and 4, mixed, 6,000 off by ~3e-3         3,457 / 6,963 / 2,156 us  (max_edge 1e-2)
+// The stack is what a lane keeps (576 bytes of layers, 1.6 KB with the calls' frames; 7.4 KB with whole
+// layers per lane): the context reserves it for every resident thread, 156 MiB (1,866 MiB).
 #include "invert_core.cuh"
 
 namespace gnurbs {
@@ -38,16 +44,23 @@ using namespace inv;
 constexpr int kQtMax = 64;     // nodes per layer (NODE_MAX_SIZE)
 constexpr int kQtLayers = 60;
 constexpr int kPortion = 128;   // queries a warp takes at a time, at most
-constexpr int kLaneCps = 512;   // control points of a node a lane scans alone
+// Nodes of a layer that a lane keeps.  4 / 8 / 16: 26.5 / 23.6 / 20.0 ms on 200,000 points off the 64x64
+// surface, 128 / 109 / 90 ms on a biquadratic one, but 16 reserve 352 MiB of local memory instead of 156.
+constexpr int kLaneNodes = 8;
+// Cost of a warp's scan of a node besides its control points, in control points of a lane's scan.  700x700
+// net, 500 points off by ~2e-3: 2,854 / 2,766 / 2,750 / 2,847 us with 0 / 2 / 8 / 32, 4,416 with the lanes
+// alone.
+constexpr int kWarpScan = 8;
 
 struct QtWarp {
   float ru[kPortion], rv[kPortion];   // mixed: ends of the root trajectories
   unsigned char list[kPortion], end[kPortion];
-  long long rest[64];             // queries the root did not answer
+  unsigned char open[kPortion];       // the portion's queries that the root did not answer
+  long long rest[32];                 // queries to be searched
   double node[2][kQtMax + 4][4];  // two layers: lb.u, lb.v, rt.u, rt.v
   int code[2][kQtMax + 4];        // index of the node's precomputed box, -1 when it has none
   double su[kQtMax], sv[kQtMax], sr[kQtMax];
-  unsigned char pass[kQtMax], ok[kQtMax];
+  unsigned char pass[kQtMax], ok[kQtMax], owner[32];
 };
 
 __device__ __forceinline__ int knot_span(const int* knot_idx, const double* b, int ns, double x) {
@@ -87,8 +100,8 @@ __device__ int split_type(const SurfDev& s, const double* nd, double max_edge) {
 // and 256x256 nets, the FP32 lengths err by at most 1.4e-4 of themselves, so both give the same
 // decision; the FP32 one costs a fraction of the FP64 work (the FP64 split types took most of a
 // launch).
-template <class Eval>
-__device__ int split_type_fast(const SurfDev& s, const Eval& ev, const double* nd, double max_edge) {
+template <int MODE, class Eval>
+__device__ __noinline__ int split_type_fast(const SurfDev& s, const Eval& ev, const double* nd, double max_edge) {
   const double iu = (nd[2] - nd[0]) / 4, iv = (nd[3] - nd[1]) / 4;
   float ul = 0, vl = 0;
   bool exact = false;
@@ -161,6 +174,16 @@ __device__ __forceinline__ void node_box(const SurfDev& s, const CpRange& r, int
     }
   }
 }
+// The same by the whole warp: every lane's result is the node's box.
+__device__ __forceinline__ void warp_box(const SurfDev& s, const CpRange& r, long long* mn, long long* mx) {
+  node_box(s, r, threadIdx.x & 31, 32, mn, mx);
+  for (int o = 16; o > 0; o >>= 1)
+    for (int c = 0; c < 3; ++c) {
+      const long long a = __shfl_xor_sync(0xffffffffu, mn[c], o), b = __shfl_xor_sync(0xffffffffu, mx[c], o);
+      mn[c] = a < mn[c] ? a : mn[c];
+      mx[c] = b > mx[c] ? b : mx[c];
+    }
+}
 __device__ __forceinline__ double key_value(long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
@@ -168,6 +191,54 @@ __device__ __forceinline__ bool box_holds(const double* mn, const double* mx, do
                                           double max_edge) {
   return px >= mn[0] - max_edge && px <= mx[0] + max_edge && py >= mn[1] - max_edge && py <= mx[1] + max_edge &&
          pz >= mn[2] - max_edge && pz <= mx[2] + max_edge;
+}
+// Whether the box of each lane's node (of the lanes with `have`) holds the lane's point.  The nodes
+// without a precomputed box are scanned by their lanes, or one after the other by the whole warp where
+// that is less work.
+__device__ __forceinline__ bool lane_box_holds(const SurfDev& s, const double* __restrict__ qtbox, bool have,
+                                               const double* nd, int code, double px, double py, double pz,
+                                               double max_edge) {
+  const unsigned FULL = 0xffffffffu;
+  const bool scan = have && code < 0;
+  double mn[3], mx[3];
+  if (have && !scan) {  // the top levels' boxes, written with the surface
+    const double* b = qtbox + 6 * code;
+    for (int c = 0; c < 3; ++c) {
+      mn[c] = b[c];
+      mx[c] = b[3 + c];
+    }
+  }
+  unsigned left = __ballot_sync(FULL, scan);
+  if (left) {
+    CpRange r = {0, 0, 1, 0};
+    if (scan) r = cp_range(s, nd);
+    const unsigned c = (unsigned)(r.cnt < 0x100000 ? r.cnt : 0x100000);
+    const unsigned longest = __reduce_max_sync(FULL, c);
+    const unsigned together = __reduce_add_sync(FULL, scan ? c / 32 + kWarpScan : 0u);
+    long long kn[3], kx[3];
+    if (longest <= together) {
+      if (scan) node_box(s, r, 0, 1, kn, kx);
+    } else {
+      for (; left; left &= left - 1) {
+        const int j = __ffs(left) - 1;
+        const CpRange rj = {__shfl_sync(FULL, r.i0, j), __shfl_sync(FULL, r.j0, j), __shfl_sync(FULL, r.nb, j),
+                            __shfl_sync(FULL, r.cnt, j)};
+        long long an[3], ax[3];
+        warp_box(s, rj, an, ax);
+        if ((threadIdx.x & 31) == j)
+          for (int k = 0; k < 3; ++k) {
+            kn[k] = an[k];
+            kx[k] = ax[k];
+          }
+      }
+    }
+    if (scan)
+      for (int k = 0; k < 3; ++k) {
+        mn[k] = key_value(kn[k]);
+        mx[k] = key_value(kx[k]);
+      }
+  }
+  return have && box_holds(mn, mx, px, py, pz, max_edge);
 }
 // children of a node split by type t (1 V, 2 U, 3 both), in the reference's order; returns their number
 __device__ __forceinline__ int put_children(int type, const double* nd, int pc, double* o, int* oc) {
@@ -253,124 +324,28 @@ __device__ __noinline__ bool node_trajectory(const SurfDev& s, const SpanTables<
   }
 }
 
-// One lane searches one query's tree from the root's children on (the root passed and had no
-// result).  Returns the status, or -1 when the search meets a node of more than kLaneCps control
-// points (it is then the warp's).
-template <int P, int Q, int MODE>
-__device__ __noinline__ int quadtree_lane(const SurfDev& s, const SpanTables<kSmemSpans>& sm, const double* __restrict__ qtbox,
-                             int root_type, double px, double py, double pz, double max_edge, double& ou, double& ov,
-                             double& orr) {
-  double node[2][kQtMax][4];
-  int code[2][kQtMax];
-  double ru[kQtMax], rv[kQtMax], rr[kQtMax];
-  const StagedEval<P, Q, kSmemSpans> ev{sm};
-  const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
-  int cur = 0, size = put_children(root_type, root, 0, node[0][0], code[0]);
-  for (int layer = 1; layer < kQtLayers && size > 0; ++layer) {
-    unsigned long long pass = 0;
-    for (int i = 0; i < size; ++i) {
-      const double* nd = node[cur][i];
-      double mn[3], mx[3];
-      if (code[cur][i] >= 0) {  // the top levels' boxes, written with the surface
-        const double* b = qtbox + 6 * code[cur][i];
-        for (int c = 0; c < 3; ++c) {
-          mn[c] = b[c];
-          mx[c] = b[3 + c];
-        }
-      } else {
-        const CpRange r = cp_range(s, nd);
-        if (r.cnt > kLaneCps) return -1;
-        long long kn[3], kx[3];
-        node_box(s, r, 0, 1, kn, kx);
-        for (int c = 0; c < 3; ++c) {
-          mn[c] = key_value(kn[c]);
-          mx[c] = key_value(kx[c]);
-        }
-      }
-      if (box_holds(mn, mx, px, py, pz, max_edge)) pass |= 1ull << i;
-    }
-    int nr = 0;
-    for (unsigned long long m = pass; m; m &= m - 1) {
-      const double* nd = node[cur][__ffsll((long long)m) - 1];
-      double u = (nd[0] + nd[2]) / 2, v = (nd[1] + nd[3]) / 2, r;
-      if (node_trajectory<P, Q, MODE>(s, sm, px, py, pz, max_edge, u, v, r)) {
-        ru[nr] = u;
-        rv[nr] = v;
-        rr[nr] = r;
-        ++nr;
-      }
-    }
-    if (nr > 0) {  // the layer's closest result (ties: the lower node)
-      int best = 0, status = 0;
-      for (int i = 1; i < nr; ++i)
-        if (rr[i] < rr[best]) best = i;
-      for (int i = 0; i < nr; ++i)
-        if (i != best && rr[i] <= rr[best] * (1 + 1e-6) + 1e-12 &&
-            (fabs(ru[i] - ru[best]) > 1e-7 || fabs(rv[i] - rv[best]) > 1e-7))
-          status = 1;
-      ou = ru[best];
-      ov = rv[best];
-      orr = rr[best];
-      return status;
-    }
-    int total = 0;
-    for (unsigned long long m = pass; m; m &= m - 1) {
-      const int i = __ffsll((long long)m) - 1;
-      const int type = split_type_fast(s, ev, node[cur][i], max_edge);
-      const int nch = type == 3 ? 4 : (type == 0 ? 0 : 2);
-      if (total + nch > kQtMax) return 3;  // layer overflow: unanswered
-      put_children(type, node[cur][i], code[cur][i], node[cur ^ 1][total], code[cur ^ 1] + total);
-      total += nch;
-    }
-    cur ^= 1;
-    size = total;
-  }
-  return 3;
-}
-
-// The whole warp searches one query's tree from the root's children on (the root passed and had no
-// result): a node's control-point box is reduced by the warp, the passing nodes' trajectories and
-// splits run one per lane.
+// The whole warp searches one query's tree from layer `layer` on, whose `size` nodes are in w.node[0] and
+// w.code[0] (no layer before had a result): a node's control-point box is reduced by the warp, the
+// passing nodes' trajectories and splits run one per lane.
 template <int P, int Q, int MODE>
 __device__ __noinline__ void quadtree_query(const SurfDev& s, const SpanTables<kSmemSpans>& sm, QtWarp& w,
-                               const double* __restrict__ qtbox, const double* __restrict__ Pq, int64_t qi,
-                               int root_type, double max_edge, double* __restrict__ uv_out, int* __restrict__ st_out, double* __restrict__ res_out) {
+                                            const double* __restrict__ qtbox, const double* __restrict__ Pq,
+                                            int64_t qi, int layer, int size, double max_edge,
+                                            double* __restrict__ uv_out, int* __restrict__ st_out,
+                                            double* __restrict__ res_out) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const double px = Pq[3 * qi], py = Pq[3 * qi + 1], pz = Pq[3 * qi + 2];
   const StagedEval<P, Q, kSmemSpans> ev{sm};
   int cur = 0, status = 3;
-  const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
-  int size = root_type == 3 ? 4 : (root_type == 0 ? 0 : 2);
   double ou = __longlong_as_double(0x7ff8000000000000ll), ov = ou, orr = ou;
-  if (lane == 0) put_children(root_type, root, 0, w.node[0][0], w.code[0]);
-  __syncwarp();
-  for (int layer = 1; layer < kQtLayers && size > 0; ++layer) {
-    // ---- control-point boxes (BoundingBoxCheck), one node at a time, the warp striding over it
-    for (int i = 0; i < size; ++i) {
-      const double* nd = w.node[cur][i];
-      double mn[3], mx[3];
-      if (w.code[cur][i] >= 0) {  // the top levels' boxes, written with the surface
-        const double* b = qtbox + 6 * w.code[cur][i];
-        for (int c = 0; c < 3; ++c) {
-          mn[c] = b[c];
-          mx[c] = b[3 + c];
-        }
-      } else {
-        long long kn[3], kx[3];
-        node_box(s, cp_range(s, nd), lane, 32, kn, kx);
-        for (int o = 16; o > 0; o >>= 1)
-          for (int c = 0; c < 3; ++c) {
-            const long long a = __shfl_xor_sync(FULL, kn[c], o), b = __shfl_xor_sync(FULL, kx[c], o);
-            kn[c] = a < kn[c] ? a : kn[c];
-            kx[c] = b > kx[c] ? b : kx[c];
-          }
-        for (int c = 0; c < 3; ++c) {
-          mn[c] = key_value(kn[c]);
-          mx[c] = key_value(kx[c]);
-        }
-      }
-      if (lane == 0) w.pass[i] = box_holds(mn, mx, px, py, pz, max_edge) ? 1 : 0;
+  for (; layer < kQtLayers && size > 0; ++layer) {
+    // ---- control-point boxes (BoundingBoxCheck), a node per lane
+    for (int base = 0; base < size; base += 32) {
+      const int i = base + lane;
+      const int k = i < size ? i : 0;
+      const bool held = lane_box_holds(s, qtbox, i < size, w.node[cur][k], w.code[cur][k], px, py, pz, max_edge);
+      if (i < size) w.pass[i] = held ? 1 : 0;
     }
     __syncwarp();
     // ---- trajectories of the passing nodes, one per lane
@@ -407,7 +382,7 @@ __device__ __noinline__ void quadtree_query(const SurfDev& s, const SpanTables<k
     for (int r = 0; r < 2; ++r) {
       const int i = lane + 32 * r;
       if (i < size && w.pass[i]) {
-        typ[r] = split_type_fast(s, ev, w.node[cur][i], max_edge);
+        typ[r] = split_type_fast<MODE>(s, ev, w.node[cur][i], max_edge);
         nch[r] = typ[r] == 3 ? 4 : (typ[r] == 0 ? 0 : 2);
       }
     }
@@ -440,6 +415,157 @@ __device__ __noinline__ void quadtree_query(const SurfDev& s, const SpanTables<k
   __syncwarp();
 }
 
+// The warp searches up to 32 queries' trees, a query per lane, from the root's children on (the root
+// passed and had no result), layer by layer.  A lane keeps its query's layer (kLaneNodes nodes) and scans
+// the control points of its nodes; the trajectories and the splits of all the lanes' passing nodes are
+// one list of tasks, which the lanes take 32 at a time, so a query with several passing nodes does not
+// run them one after the other on its lane.  A query whose layer is wider is searched on by the whole
+// warp (quadtree_query).  rest: the queries; cnt: their number.
+template <int P, int Q, int MODE>
+__device__ __forceinline__ void quadtree_search(const SurfDev& s, const SpanTables<kSmemSpans>& sm, QtWarp& w,
+                                                const double* __restrict__ qtbox, const double* __restrict__ Pq,
+                                                const long long* rest, int cnt, int root_type, double max_edge,
+                                                double* __restrict__ uv_out, int* __restrict__ st_out,
+                                                double* __restrict__ res_out) {
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  const StagedEval<P, Q, kSmemSpans> ev{sm};
+  double node[2][kLaneNodes][4];
+  int code[2][kLaneNodes];
+  const long long q = lane < cnt ? rest[lane] : 0;
+  bool open = lane < cnt;  // not answered yet
+  int cur = 0, size = 0;
+  if (open) {
+    const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
+    size = put_children(root_type, root, 0, node[0][0], code[0]);
+  }
+  auto answer = [&](int status, double u, double v, double r) {
+    uv_out[2 * q] = u;
+    uv_out[2 * q + 1] = v;
+    st_out[q] = status;
+    res_out[q] = r;
+    open = false;
+  };
+  // the position of this lane's first task when each lane has as many as `mask` has bits, and the total
+  auto place = [&](unsigned mask, int& total) {
+    const int k = __popc(mask);
+    int incl = k;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += t;
+    }
+    total = __shfl_sync(FULL, incl, 31);
+    return incl - k;
+  };
+  for (int layer = 1; layer < kQtLayers && __any_sync(FULL, size > 0); ++layer) {
+    // ---- control-point boxes (BoundingBoxCheck)
+    unsigned pass = 0;
+    for (int i = 0; __any_sync(FULL, i < size); ++i) {
+      const int k = i < size ? i : 0;
+      if (lane_box_holds(s, qtbox, i < size, node[cur][k], code[cur][k], Pq[3 * q], Pq[3 * q + 1], Pq[3 * q + 2],
+                         max_edge))
+        pass |= 1u << i;
+    }
+    // ---- trajectories of the passing nodes; the converged ones' (u, v, residual) in node order replace
+    // the layer before this one
+    int total, nr = 0;
+    int first = place(pass, total);
+    for (int base = 0; base < total; base += 32) {
+      int t = first - base;
+      for (unsigned m = pass; m; m &= m - 1, ++t)
+        if (t >= 0 && t < 32) {
+          const double* nd = node[cur][__ffs(m) - 1];
+          w.owner[t] = (unsigned char)lane;
+          w.su[t] = (nd[0] + nd[2]) / 2;
+          w.sv[t] = (nd[1] + nd[3]) / 2;
+        }
+      __syncwarp();
+      const bool task = base + lane < total;
+      const long long qo = __shfl_sync(FULL, q, task ? w.owner[lane] : 0);
+      if (task) {
+        double u = w.su[lane], v = w.sv[lane], rr = 0;
+        w.ok[lane] = node_trajectory<P, Q, MODE>(s, sm, Pq[3 * qo], Pq[3 * qo + 1], Pq[3 * qo + 2], max_edge, u, v, rr);
+        w.su[lane] = u;
+        w.sv[lane] = v;
+        w.sr[lane] = rr;
+      }
+      __syncwarp();
+      t = first - base;
+      for (unsigned m = pass; m; m &= m - 1, ++t)
+        if (t >= 0 && t < 32 && w.ok[t]) {
+          double* o = node[cur ^ 1][nr++];
+          o[0] = w.su[t];
+          o[1] = w.sv[t];
+          o[2] = w.sr[t];
+        }
+      __syncwarp();
+    }
+    // ---- the layer's closest result (ties: the lower node), if any
+    if (nr > 0) {
+      const double(*o)[4] = node[cur ^ 1];
+      int best = 0, status = 0;
+      for (int i = 1; i < nr; ++i)
+        if (o[i][2] < o[best][2]) best = i;
+      for (int i = 0; i < nr; ++i)
+        if (i != best && o[i][2] <= o[best][2] * (1 + 1e-6) + 1e-12 &&
+            (fabs(o[i][0] - o[best][0]) > 1e-7 || fabs(o[i][1] - o[best][1]) > 1e-7))
+          status = 1;
+      answer(status, o[best][0], o[best][1], o[best][2]);
+      pass = 0;
+    }
+    // ---- the passing nodes' split types (getSplitType), two bits each
+    unsigned types = 0;
+    first = place(pass, total);
+    for (int base = 0; base < total; base += 32) {
+      int t = first - base;
+      for (unsigned m = pass; m; m &= m - 1, ++t)
+        if (t >= 0 && t < 32) {
+          const double* nd = node[cur][__ffs(m) - 1];
+          put_node(w.node[0][t], nd[0], nd[1], nd[2], nd[3]);
+        }
+      __syncwarp();
+      if (base + lane < total) w.ok[lane] = (unsigned char)split_type_fast<MODE>(s, ev, w.node[0][lane], max_edge);
+      __syncwarp();
+      t = first - base;
+      for (unsigned m = pass; m; m &= m - 1, ++t)
+        if (t >= 0 && t < 32) types |= (unsigned)w.ok[t] << (2 * (__ffs(m) - 1));
+      __syncwarp();
+    }
+    // ---- their children, in node order
+    auto children = [&](int i) {
+      const unsigned type = types >> (2 * i) & 3u;
+      return type == 3 ? 4 : (type == 0 ? 0 : 2);
+    };
+    int many = 0;
+    for (unsigned m = pass; m; m &= m - 1) many += children(__ffs(m) - 1);
+    if (many > kQtMax) many = 0;  // layer overflow: unanswered
+    auto put_layer = [&](double (*o)[4], int* oc) {
+      int at = 0;
+      for (unsigned m = pass; m; m &= m - 1) {
+        const int i = __ffs(m) - 1;
+        at += put_children((int)(types >> (2 * i) & 3u), node[cur][i], code[cur][i], o[at], oc + at);
+      }
+    };
+    const bool wide = many > kLaneNodes;
+    if (many > 0 && !wide) put_layer(node[cur ^ 1], code[cur ^ 1]);
+    for (unsigned wm = __ballot_sync(FULL, wide); wm; wm &= wm - 1) {
+      const int j = __ffs(wm) - 1;
+      if (lane == j) {
+        put_layer(w.node[0], w.code[0]);
+        open = false;
+      }
+      __syncwarp();
+      quadtree_query<P, Q, MODE>(s, sm, w, qtbox, Pq, __shfl_sync(FULL, q, j), layer + 1, __shfl_sync(FULL, many, j),
+                                 max_edge, uv_out, st_out, res_out);
+    }
+    size = wide ? 0 : many;
+    cur ^= 1;
+  }
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  if (open) answer(3, nan, nan, nan);
+  __syncwarp();
+}
+
 // Register budget: 4 CTAs per SM (128 registers); the run-time degrees' variant 2.
 template <int P, int Q, int MODE>
 __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
@@ -460,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
   const double cu = (s.dom_u0 + s.dom_u1) / 2, cv = (s.dom_v0 + s.dom_v1) / 2;
   float far[4];
   far_limits(cx, far);
-  int nrest = 0, root_type = -1;
+  int nrest = 0, nopen = 0, root_type = -1;
   int64_t seen = 0;
   auto answer = [&](int64_t q, int status, double u, double v, double r) {
     uv_out[2 * q] = u;
@@ -468,49 +594,22 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
     st_out[q] = status;
     res_out[q] = r;
   };
-  // the last `cnt` queries of the queue
-  auto search = [&](int cnt) {
-    if (root_type < 0) {
-      const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
-      root_type = split_type_fast(s, ev, root, max_edge);
-    }
-    nrest -= cnt;
-    unsigned byw = cnt <= 2 ? (1u << cnt) - 1u : 0u;  // searched by the whole warp
-    if (cnt > 2) {
-      bool big = false;
-      if (lane < cnt) {
-        const int64_t q = w.rest[nrest + lane];
-        double u = nan, v = nan, r = nan;
-        const int st = quadtree_lane<P, Q, MODE>(s, sm, qtbox, root_type, Pq[3 * q], Pq[3 * q + 1], Pq[3 * q + 2],
-                                                 max_edge, u, v, r);
-        big = st < 0;
-        if (!big) answer(q, st, u, v, r);
-      }
-      byw = __ballot_sync(FULL, big);
-    }
-    for (; byw; byw &= byw - 1)
-      quadtree_query<P, Q, MODE>(s, sm, w, qtbox, Pq, w.rest[nrest + __ffs(byw) - 1], root_type, max_edge, uv_out,
-                                 st_out, res_out);
-    __syncwarp();
-  };
-  // queues the queries of the lanes with `open`, and searches a full warp's worth
-  auto queue = [&](bool open, int64_t q) {
+  // the lanes' queries k of the portion that the root did not answer
+  auto queue = [&](bool open, int k) {
     const unsigned m = __ballot_sync(FULL, open);
-    if (open) w.rest[nrest + __popc(m & lt_mask)] = q;
-    nrest += __popc(m);
-    __syncwarp();
-    if (nrest >= 32) search(32);
+    if (open) w.open[nopen + __popc(m & lt_mask)] = (unsigned char)k;
+    nopen += __popc(m);
   };
-  for (;;) {
+  for (bool last = false; !last;) {
     // this warp's share of what is left, a few queries at least
     const float fair = (float)(n - seen) * share;
     const int want = max(fair < (float)kPortion ? (int)fair + 1 : kPortion, least);
     unsigned long long a = 0;
     if (lane == 0) a = atomicAdd(counter, (unsigned long long)want);
     const int64_t q0 = (int64_t)__shfl_sync(FULL, a, 0);
-    if (q0 >= n) break;
+    last = q0 >= n;
     seen = q0 + want;
-    const int cnt = (int)(n - q0 < want ? n - q0 : want);
+    const int cnt = last ? 0 : (int)(n - q0 < want ? n - q0 : want);
     // ---- the root's box: queries outside it have no candidate
     int total = 0;
     for (int base = 0; base < cnt; base += 32) {
@@ -544,13 +643,13 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
           }
         } else {
           bool open = false;
-          const int64_t q = q0 + w.list[slot];
+          const int k = w.list[slot];
           if (end != kContinue) {
             const double r = sqrt(dist);
-            if (end == kConverged && in_domain64(cx, sd.u, sd.v, dist) && r < max_edge) answer(q, 0, sd.u, sd.v, r);
+            if (end == kConverged && in_domain64(cx, sd.u, sd.v, dist) && r < max_edge) answer(q0 + k, 0, sd.u, sd.v, r);
             else open = true;
           }
-          queue(open, q);
+          queue(open, k);
         }
         end = kContinue;
         if (next >= total && wm == FULL) break;
@@ -589,9 +688,8 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
       for (int base = 0; base < total; base += 32) {
         const int k = base + lane;
         bool open = false;
-        int64_t q = 0;
         if (k < total) {
-          q = q0 + w.list[k];
+          const int64_t q = q0 + w.list[k];
           open = true;
           if (w.end[k] == kConverged) {
             double u = w.ru[k], v = w.rv[k], r;
@@ -601,11 +699,26 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
             }
           }
         }
-        queue(open, q);
+        queue(open, k < total ? w.list[k] : 0);
       }
     }
+    __syncwarp();
+    // ---- the open queries' trees, a full warp's worth at a time
+    for (;;) {
+      const int more = min(nopen, 32 - nrest);
+      nopen -= more;
+      if (lane < more) w.rest[nrest + lane] = q0 + w.open[nopen + lane];
+      nrest += more;
+      __syncwarp();
+      if (nrest < 32 && !(last && nrest > 0)) break;
+      if (root_type < 0) {
+        const double root[4] = {s.dom_u0, s.dom_v0, s.dom_u1, s.dom_v1};
+        root_type = split_type_fast<MODE>(s, ev, root, max_edge);
+      }
+      quadtree_search<P, Q, MODE>(s, sm, w, qtbox, Pq, w.rest, nrest, root_type, max_edge, uv_out, st_out, res_out);
+      nrest = 0;
+    }
   }
-  if (nrest > 0) search(nrest);
 }
 
 template <int P, int Q, int MODE>
