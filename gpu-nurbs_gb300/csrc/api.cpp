@@ -402,8 +402,6 @@ int nurbs_build_tree(nurbs_surface_t s, int levels, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   CUDA_TRY(launch_nodes(s->dev, st), "tree launch");
   CUDA_TRY(launch_centre_ders(s->dev, st), "seed-centre derivatives");
-  CUDA_TRY(cudaMemcpyAsync(&s->dev.seeds, s->dev.cd32 + 9 * kTreeNodes, sizeof(float), cudaMemcpyDeviceToHost, st),
-           "average candidates");
   CUDA_TRY(cudaStreamSynchronize(st), "tree sync");
   s->tree_built = true;
   return NURBS_OK;

@@ -8,9 +8,11 @@
 // NeedDivide (kernel.cu:859-878).
 //
 // Two launches.  k_nodes: one CTA per node evaluates the node's samples and reduces them to the
-// unclipped box, the unclipped normal box and the control-point box; a node's samples do not
-// depend on its parent, so both levels run at once (the quadtree boxes are further CTAs of the same
-// launch).  k_nodes_finish: a warp per node clips to the root and writes the records.
+// unclipped box, the unclipped normal box and the control-point box, in nodebox; a node's samples do
+// not depend on its parent, so both levels run at once (the quadtree boxes are further CTAs of the same
+// launch).  k_nodes_finish: a warp per node clips to the root and writes the records.  Only final values
+// are written to what the queries read, so a rebuild, which repeats them, does not disturb queries on
+// other streams.
 //
 // What bounds it: FP64 arithmetic in the reference's order.  An FP64 instruction of a warp takes 64
 // clocks here whatever its active lanes, so the build is a question of how few of them follow one
@@ -111,9 +113,8 @@ __device__ __forceinline__ void hull_of(const SurfDev& s, int a0, int a1, int b0
     }
 }
 
-// The samples of node k (0: root, 1 + bx*8 + by: its children): unclipped box into tree[k]; CONES:
-// also the unclipped normal box into nbox[k], the lattice points, and the control-point box as six
-// doubles in the node's cone record, where k_nodes_finish takes it from.
+// The samples of node k (0: root, 1 + bx*8 + by: its children): its unclipped box into nodebox; CONES:
+// also its unclipped normal box and control-point box there, and the lattice points.
 //
 // Normal cones (the projection's culling data): the normal N = Su x Sv and its second derivatives at
 // the same samples, the normal box widened by the box tree's bound K applied to N.
@@ -326,19 +327,14 @@ __device__ __forceinline__ void node_samples(const SurfDev& s, int k) {
     // sqrt(3): kernel.cu:574
     const double K = (shfl(acc, 0) + 2 * shfl(acc, 1) + shfl(acc, 2)) * 1.7320508075688772 / den;
     const double KN = (shfl(acc, 3) + 2 * shfl(acc, 4) + shfl(acc, 5)) * 1.7320508075688772 / den;
-    TreeNodeDev& n = s.tree[k];
-    if (lane >= 6 && lane < 9) n.rt[j] = acc + K;
-    if (lane >= 9 && lane < 12) n.lb[j] = acc - K;
+    double* box = s.nodebox + 6 * k;
+    if (lane >= 6 && lane < 9) box[3 + j] = acc + K;
+    if (lane >= 9 && lane < 12) box[j] = acc - K;
     if (CONES) {
-      if (lane >= 12 && lane < 15) s.nbox[6 * k + 3 + j] = acc + KN;
-      if (lane >= 15 && lane < 18) s.nbox[6 * k + j] = acc - KN;
-      if (lane >= 18 && lane < 24) reinterpret_cast<double*>(s.cone + kConeStride * k)[lane - 18] = acc;
-    }
-    if (lane == 0) {
-      n.uv_lb[0] = bx * uunit;
-      n.uv_lb[1] = by * uunit;
-      n.uv_rt[0] = (bx + 1) * uunit;
-      n.uv_rt[1] = (by + 1) * uunit;
+      double *nbox = box + 6 * kTreeNodes, *hull = nbox + 6 * kTreeNodes;
+      if (lane >= 12 && lane < 15) nbox[3 + j] = acc + KN;
+      if (lane >= 15 && lane < 18) nbox[j] = acc - KN;
+      if (lane >= 18 && lane < 24) hull[lane - 18] = acc;
     }
   }
 }
@@ -353,28 +349,39 @@ __device__ __forceinline__ float round_up(double x) { return __double2float_ru(x
 template <bool CONES>
 __device__ __forceinline__ void node_finish(const SurfDev& s, int k) {
   const int lane = threadIdx.x & 31;
-  const TreeNodeDev root = s.tree[0];  // the root's box is not clipped: k_nodes wrote its final values
-  TreeNodeDev n = s.tree[k];
+  const unsigned bx = k == 0 ? 0u : (unsigned)(k - 1) / kGap, by = k == 0 ? 0u : (unsigned)(k - 1) % kGap;
+  const double uunit = k == 0 ? 1.0 : 1.0 / kGap;
+  const double *box0 = s.nodebox, *nbox0 = box0 + 6 * kTreeNodes, *hull0 = nbox0 + 6 * kTreeNodes;  // the root's
+  TreeNodeDev root, n;
+  for (int c = 0; c < 3; ++c) {
+    root.lb[c] = box0[c];
+    root.rt[c] = box0[3 + c];
+    n.lb[c] = box0[6 * k + c];
+    n.rt[c] = box0[6 * k + 3 + c];
+  }
+  n.uv_lb[0] = bx * uunit;
+  n.uv_lb[1] = by * uunit;
+  n.uv_rt[0] = (bx + 1) * uunit;
+  n.uv_rt[1] = (by + 1) * uunit;
   const bool built = k == 0 || need_divide(root);  // children of a flat root are not built
   double nb[6] = {0, 0, 0, 0, 0, 0}, hb[6] = {0, 0, 0, 0, 0, 0};
   if (CONES)
     for (int c = 0; c < 6; ++c) {
-      nb[c] = s.nbox[6 * k + c];
-      hb[c] = reinterpret_cast<const double*>(s.cone + kConeStride * k)[c];
+      nb[c] = nbox0[6 * k + c];
+      hb[c] = hull0[6 * k + c];
     }
   if (k > 0)
     for (int c = 0; c < 3; ++c) {  // min/max(TreeNode) against the parent (kernel.cu:606-611, 885-901)
       n.rt[c] = fmin(n.rt[c], root.rt[c]);
       n.lb[c] = fmax(n.lb[c], root.lb[c]);
       if (CONES) {
-        nb[c] = fmax(nb[c], s.nbox[c]);
-        nb[3 + c] = fmin(nb[3 + c], s.nbox[3 + c]);
+        nb[c] = fmax(nb[c], nbox0[c]);
+        nb[3 + c] = fmin(nb[3 + c], nbox0[3 + c]);
       }
     }
-  __syncwarp();
   if (lane == 0) {
     if (!built) n = TreeNodeDev{};
-    if (k > 0) s.tree[k] = n;
+    s.tree[k] = n;
     s.divided[k] = built && need_divide(n) ? 1 : 0;
     s.built[k] = built ? 1 : 0;
   }
@@ -385,7 +392,7 @@ __device__ __forceinline__ void node_finish(const SurfDev& s, int k) {
     if (lane < kConeStride) rec[lane] = 0;
     return;
   }
-  if (k > 0 && lane == 0)
+  if (lane == 0)
     for (int c = 0; c < 6; ++c) s.nbox[6 * k + c] = nb[c];
   // the node's own box where it is narrower
   double xb[6];

@@ -54,7 +54,10 @@ constexpr int kQuadtreeBoxes = ((1 << (2 * kQuadtreeDepth)) - 1) / 3;  // 341
 //                                    FP32 relative to org: distance bounds and projection seeds
 //   qtbox[341][6]                    control-point boxes of the quadtree inversion's square nodes of
 //                                    depth 0..4, written with the tree
-// (pooled surfaces, which are only inverted and evaluated, have no nbox, cone, lattice and qtbox)
+//   nodebox[3][65][6]                scratch of the node kernels: the nodes' unclipped boxes, normal boxes
+//                                    and control-point boxes
+// (pooled surfaces, which are only inverted and evaluated, have no nbox, cone, lattice and qtbox, and
+// their nodebox is the first plane only, in the place of cd64, which is written later)
 struct SurfDev {
   int p, q, nu, nv;
   int ns_u, ns_v;
@@ -90,6 +93,7 @@ struct SurfDev {
   float* cd32;            // seed-centre derivatives (see above)
   float seeds;            // single surfaces: a host copy of cd32[65*9] (0 before the tree is built)
   double* cd64;
+  double* nodebox;        // the conversion's unclipped boxes (see above)
   double* nbox;           // normal cones (see above)
   float* cone;
   float* lattice;

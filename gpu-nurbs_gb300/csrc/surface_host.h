@@ -69,7 +69,7 @@ struct SurfaceHost {
   size_t o_bu, o_bv, o_idu, o_idv, o_bu32, o_bv32, o_idu32, o_idv32, o_iu, o_iv, o_gu, o_gv, o_ku, o_kv, o_cps, o_w, o_tree,
       o_div, o_built, in_bytes;
   // offsets inside the computed part
-  size_t o_m64, o_m32, o_bas_u, o_bas_v, o_cd32, o_cd64, o_nbox, o_cone, o_lat, o_qtb, out_bytes;
+  size_t o_m64, o_m32, o_bas_u, o_bas_v, o_cd32, o_cd64, o_nbox, o_cone, o_lat, o_qtb, o_nodebox, out_bytes;
 };
 
 // Validates and prepares a surface given by host arrays.  Returns NURBS_OK or an error code,
@@ -151,6 +151,7 @@ inline int prepare_surface(int p, int q, int nu, int nv, const double* ku, const
     S.o_cone = take(kTreeNodes * kConeStride * 4);
     S.o_lat = take(kTreeNodes * kPts * kPts * 3 * 4);
     S.o_qtb = take(kQuadtreeBoxes * 6 * 8);
+    S.o_nodebox = take(3 * kTreeNodes * 6 * 8);
   }
   S.out_bytes = off;
   return NURBS_OK;
@@ -217,7 +218,9 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.basis_v = (double*)(out_dev + S.o_bas_v);
   d.cd32 = (float*)(out_dev + S.o_cd32);
   d.cd64 = (double*)(out_dev + S.o_cd64);
+  d.nodebox = d.cd64;
   if (S.culling) {
+    d.nodebox = (double*)(out_dev + S.o_nodebox);
     d.nbox = (double*)(out_dev + S.o_nbox);
     d.cone = (float*)(out_dev + S.o_cone);
     d.lattice = (float*)(out_dev + S.o_lat);

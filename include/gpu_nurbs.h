@@ -184,7 +184,8 @@ int nurbs_evaluate_random(const double* uv_dev, double* xyz_dev, int64_t n, cons
 /* ------------------------------------------------ stage c: subdivision tree / culling */
 /* (Re)builds the tree: GetPoints + GetSecondDerivatives + Max_Sequential_Addressing_Shared
  * + TightBoundingBox for levels 0..levels-1 (src/main.cu:280-309).  Only levels == 2 (the
- * reference's setting) is supported. */
+ * reference's setting) is supported.  nurbs_surface_create has built it; a rebuild writes the same
+ * values again, so queries of the surface may run meanwhile on other streams and threads. */
 int nurbs_build_tree(nurbs_surface_t s, int levels, void* stream);
 /* Copies the tree to host memory in the reference TreeNode order (kernel.cuh:30-39):
  * per node 10 doubles {uv.lb.x, uv.lb.y, uv.rt.x, uv.rt.y, lb.x, lb.y, lb.z, rt.x, rt.y, rt.z},
