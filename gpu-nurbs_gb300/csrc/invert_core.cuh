@@ -105,25 +105,19 @@ struct Ctx {
   const double* m64;
   int p, q;
   double dom_u0, dom_u1, dom_v0, dom_v1;
-  bool unit_range;   // both knot ranges are 1
-  double iru, irv;   // 1 / knot range, set when they are not
+  double iru, irv;   // 1 / knot range
 };
-__device__ __forceinline__ void set_range(const SurfDev& s, Ctx& c) {
-  const long long one = __double_as_longlong(1.0);
-  c.unit_range = __double_as_longlong(s.range_u) == one && __double_as_longlong(s.range_v) == one;
-  c.iru = c.irv = 1.0;
-  if (!c.unit_range) {
-    c.iru = 1.0 / s.range_u;
-    c.irv = 1.0 / s.range_v;
-  }
-}
 
 // |S - P|^2 at (u - du, v - dv) from r = S - P, Su, Sv at (u, v): S(u - du, v - dv) = S - Su du -
 // Sv dv + O(|S''| 1e-20) for the steps a seed ends with (1e-10 at most), below the rounding of S
 // itself.  Su and Sv are scaled by the knot range (kernel.cu:167), so the steps are divided by it.
+// BRANCH: only where it is not 1, for the loops in which some lane ends in nearly every turn (the FP64
+// multiplications are 0.7 % of an FP64 iteration; the branch costs the pool's final steps 1 %).
+template <bool BRANCH>
 __device__ __forceinline__ double dist2_after(const Ctx& c, const v3<double>& r, const v3<double>& Su,
                                               const v3<double>& Sv, double du, double dv) {
-  if (!c.unit_range) {
+  const long long one = 0x3ff0000000000000ll;
+  if (!BRANCH || __double_as_longlong(c.iru) != one || __double_as_longlong(c.irv) != one) {
     du *= c.iru;
     dv *= c.irv;
   }
@@ -203,7 +197,7 @@ __device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, dou
   st.v -= dv;
   const double step = fast::max_abs(du, dv);
   if ((st.newton && fast::le_nonneg(step, kTolNewton64)) || fast::le_nonneg(step, kTolAny64)) {
-    dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
+    dist2 = dist2_after<true>(c, r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   st.prev = step;
@@ -302,7 +296,7 @@ __device__ __forceinline__ int final_step(const Ctx& c, const Eval& ev, double p
   f.u -= du;
   f.v -= dv;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
-    const double dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
+    const double dist2 = dist2_after<false>(c, r, d.Su, d.Sv, du, dv);
     res = sqrt(dist2);
     return in_domain64(c, f.u, f.v, dist2) ? kConverged : kFailed;
   }
@@ -490,7 +484,7 @@ __device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& s
     cx.p = s.p;
     cx.q = s.q;
     cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
-    set_range(s, cx);
+    cx.iru = s.inv_range_u; cx.irv = s.inv_range_v;
   }
 }
 

@@ -36,7 +36,8 @@ __device__ __forceinline__ Ctx global_ctx(const SurfDev& s) {
   cx.dom_u1 = s.dom_u1;
   cx.dom_v0 = s.dom_v0;
   cx.dom_v1 = s.dom_v1;
-  set_range(s, cx);
+  cx.iru = s.inv_range_u;
+  cx.irv = s.inv_range_v;
   return cx;
 }
 

@@ -175,7 +175,7 @@ __device__ __forceinline__ int project_advance(const Ctx& c, const fast::SDer<T>
   st.trial = false;
   const T du = st.u - st.un, dv = st.v - st.vn;
   if (moved_to()) {
-    if constexpr (!kFp32) dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
+    if constexpr (!kFp32) dist2 = dist2_after<true>(c, r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   return ++st.it >= kMaxIterProj ? kFailed : kContinue;
@@ -280,7 +280,7 @@ __device__ __forceinline__ int project_polish_step(const Ctx& c, const Eval& ev,
   f.u = un;
   f.v = vn;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewtonProj)) {
-    const double dist2 = dist2_after(c, r, d.Su, d.Sv, du, dv);
+    const double dist2 = dist2_after<false>(c, r, d.Su, d.Sv, du, dv);
     res = sqrt(dist2);
     return fast::is_finite(dist2) ? kConverged : kFailed;
   }
