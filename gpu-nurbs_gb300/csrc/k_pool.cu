@@ -165,6 +165,22 @@ cudaError_t launch_eval_pool(const SurfDev* table, const InvTile* tiles, int nti
   return cudaGetLastError();
 }
 
+int pool_ctas_per_sm(int precision) {
+  static int cached[2][64] = {};
+  const int mode = precision == 1 ? 1 : 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  int& c = cached[mode][dev];
+  if (!c) {
+    int fit = 0;
+    if (mode) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_invert_pool_cta<kModeMixed>, kThreads, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_invert_pool_cta<kModeFP64>, kThreads, 0);
+    c = fit > 0 ? fit : 1;
+  }
+  return c;
+}
+
 cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int ntiles, int* counter, const double* P,
                                double* uv, int* status, double* residual, int precision, int ctas, int tile_queries,
                                cudaStream_t st) {
@@ -172,11 +188,11 @@ cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int n
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   if (ctas > ntiles) ctas = ntiles;
+  // (ctas are resident ones: at most pool_ctas_per_sm per SM)
   // Tiles per grab: small tiles together, up to kGroupQueries queries, while every resident CTA gets a
   // grab.  Larger tiles one by one: groups of 8 / 2 / 1 tiles of 128 take 41.3 / 35.8 / 32.8 ms on 600
   // surfaces with 4.4 M queries (the last groups are the launch's tail), and the same on 300 with 1 M.
-  const int resident = std::min(ctas, kCtasPerSm * 152);
-  const int group = std::max(1, std::min(ntiles / resident, kGroupQueries / tile_queries));
+  const int group = std::max(1, std::min(ntiles / ctas, kGroupQueries / tile_queries));
   if (precision == 1)
     k_invert_pool_cta<kModeMixed><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
                                                              group);

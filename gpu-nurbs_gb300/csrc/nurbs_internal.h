@@ -160,6 +160,9 @@ cudaError_t launch_span_matrices_batched(const SurfDev* table, const SpanJob* jo
 cudaError_t launch_nodes_batched(const SurfDev* table, const int* ids, int count, cudaStream_t st);
 cudaError_t launch_eval_pool(const SurfDev* table, const InvTile* tiles, int ntiles, const double* uv, int64_t n,
                              unsigned mask, double* out, cudaStream_t st);
+// CTAs of the pool's inversion kernel that an SM of the current GPU holds
+int pool_ctas_per_sm(int precision);
+// ctas: at most what the GPU holds
 cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int ntiles, int* counter,
                                const double* P, double* uv, int* status, double* residual, int precision,
                                int ctas, int tile_queries, cudaStream_t st);

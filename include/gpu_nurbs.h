@@ -305,7 +305,8 @@ const char* nurbs_pool_last_error(void);
 /* Launch configuration and persistent CTAs per SM.  tile_queries: queries of one surface
  * that a CTA takes at a time, a multiple of 32 (throughput on large batches) or at most 32 (small
  * batches spread over all SMs; fewer queries per CTA lower latency; large batches take several such
- * tiles at a time). */
+ * tiles at a time).  ctas_per_sm: 1..16; at most as many as an SM holds of the kernel are launched
+ * (4 on the GB300, the default). */
 int nurbs_pool_set_config(nurbs_pool_t pool, int tile_queries, int ctas_per_sm);
 /* Batched inversion.  Queries are grouped by surface: surface ids_host[k] owns the queries
  * [offsets_host[k], offsets_host[k+1]) of P_dev (3 doubles each); outputs are indexed like P.
@@ -319,7 +320,8 @@ int nurbs_pool_eval(nurbs_pool_t pool, int nbatch, const int* ids_host, const in
                     const double* uv_dev, int64_t n, unsigned mask, double* out_dev, void* stream);
 /* Times tile size x CTAs per SM on the batch (or its prefix of at most max_queries queries, 0 =
  * all), keeps the fastest configuration in the pool and returns it.  With cache_path, a result
- * cached for the same GPU, precision and batch signature is reused, and new results appended. */
+ * cached for the same GPU, kernel schedule, precision and batch signature is reused, and new results
+ * appended. */
 int nurbs_pool_autotune(nurbs_pool_t pool, int nbatch, const int* ids_host, const int64_t* offsets_host,
                         const double* P_dev, double* uv_dev, int* status_dev, double* residual_dev, int precision,
                         int64_t max_queries, const char* cache_path, void* stream, int* best_tile, int* best_ctas,
