@@ -51,7 +51,6 @@ constexpr int kRefill64 = 8;
 // Seeds a warp's least portion holds (least_grab).  Mixed, 32 / 64: 64x64 surface, 6,000 queries 230 /
 // 210 us; 8x8 surface, 60,000 queries 145 / 126 us; FP64 64 / 128: 50,021 queries 6.73 / 6.67 ms.
 constexpr float kGrabSeedsMixed = 64, kGrabSeeds64 = 128;
-constexpr int kSchedulers = 4 * 152;  // of the GB300: four per SM, an FP64 pipe each
 
 // Arithmetic below writes every product that feeds a sum as an explicit FMA (the translation
 // units are compiled with --fmad=false), so a seed's trajectory is the same bit for bit in

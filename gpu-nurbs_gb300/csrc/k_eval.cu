@@ -171,7 +171,6 @@ static int order_of(unsigned mask) {
 
 template <typename T, int P, int Q>
 static cudaError_t launch_pq(const SurfDev& s, const T* uv, int64_t n, unsigned mask, T* out, cudaStream_t st) {
-  constexpr int kSchedulers = 4 * 152;
   int threads = 256;
   if constexpr (sizeof(T) == 8) {
     // four lanes per point while that leaves at most one warp per scheduler, then warps of their own

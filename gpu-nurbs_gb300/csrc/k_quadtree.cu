@@ -184,9 +184,6 @@ __device__ __forceinline__ void warp_box(const SurfDev& s, const CpRange& r, lon
       mx[c] = b > mx[c] ? b : mx[c];
     }
 }
-__device__ __forceinline__ double key_value(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
-}
 __device__ __forceinline__ bool box_holds(const double* mn, const double* mx, double px, double py, double pz,
                                           double max_edge) {
   return px >= mn[0] - max_edge && px <= mx[0] + max_edge && py >= mn[1] - max_edge && py <= mx[1] + max_edge &&
@@ -234,8 +231,8 @@ __device__ __forceinline__ bool lane_box_holds(const SurfDev& s, const double* _
     }
     if (scan)
       for (int k = 0; k < 3; ++k) {
-        mn[k] = key_value(kn[k]);
-        mx[k] = key_value(kx[k]);
+        mn[k] = fast::key_value(kn[k]);
+        mx[k] = fast::key_value(kx[k]);
       }
   }
   return have && box_holds(mn, mx, px, py, pz, max_edge);

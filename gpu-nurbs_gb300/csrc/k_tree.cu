@@ -55,15 +55,6 @@ struct NodeReduce {  // per warp, by component lane: maxima and minima of S and 
   long long hull[6];
 };
 
-// Order-preserving integer image of a double (not NaN), and back.
-__device__ __forceinline__ long long order_key(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-__device__ __forceinline__ double key_value(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
-}
-
 // Maximum (or minimum) over the warp's samples of lanes of one component (lanes 4 apart), with the
 // sequential scan's result: a NaN is skipped, and of equal values the first sample's stays.
 template <bool MAX>
@@ -83,7 +74,7 @@ __device__ __forceinline__ double warp_pick(double x) {
 }
 __device__ __forceinline__ double shfl(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
 
-// Control points a0..a1 x b0..b1: order keys of their minima (0..2) and maxima (3..5) over the
+// Control points a0..a1 x b0..b1: total keys of their minima (0..2) and maxima (3..5) over the
 // elements t, t + stride, ..., reduced over the warp.
 __device__ __forceinline__ void hull_of(const SurfDev& s, int a0, int a1, int b0, int b1, int t, int stride,
                                         long long h[6]) {
@@ -98,7 +89,7 @@ __device__ __forceinline__ void hull_of(const SurfDev& s, int a0, int a1, int b0
     const double* x = s.cps + 3 * ((size_t)(a0 + row) * s.nv + (b0 + col));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const long long k = order_key(x[c]);
+      const long long k = fast::total_key(x[c]);
       h[c] = k < h[c] ? k : h[c];
       h[3 + c] = k > h[3 + c] ? k : h[3 + c];
     }
@@ -321,7 +312,7 @@ __device__ __forceinline__ void node_samples(const SurfDev& s, int k) {
         const long long o = red[w].hull[lane - 18];
         hk = lane < 21 ? (o < hk ? o : hk) : (o > hk ? o : hk);
       }
-      acc = key_value(hk);
+      acc = fast::key_value(hk);
     }
     const unsigned den = 8u * kGap * g * kGap * g;
     // sqrt(3): kernel.cu:574
@@ -482,7 +473,7 @@ __device__ __forceinline__ void quadtree_box_cta(const SurfDev& s, int code) {
     const int c = threadIdx.x;
     long long k = red[0][c];
     for (int w = 1; w < kNodeWarps; ++w) k = c < 3 ? min(k, red[w][c]) : max(k, red[w][c]);
-    s.qtbox[6 * code + c] = key_value(k);
+    s.qtbox[6 * code + c] = fast::key_value(k);
   }
 }
 __device__ __forceinline__ void quadtree_box_warp(const SurfDev& s, int code) {
@@ -490,7 +481,7 @@ __device__ __forceinline__ void quadtree_box_warp(const SurfDev& s, int code) {
   long long h[6];
   quadtree_box(s, code, threadIdx.x & 31, 32, h);
   if ((threadIdx.x & 31) == 0)
-    for (int c = 0; c < 6; ++c) s.qtbox[6 * code + c] = key_value(h[c]);
+    for (int c = 0; c < 6; ++c) s.qtbox[6 * code + c] = fast::key_value(h[c]);
 }
 
 __global__ void __launch_bounds__(kNodeThreads) k_nodes(SurfDev s) {

@@ -5,6 +5,7 @@
 
 namespace gnurbs {
 
+constexpr int kSchedulers = 4 * 152;  // of the GB300: four per SM, an FP64 pipe each
 constexpr int kMaxDegree = 7;     // p, q <= 7 (reference MAX_DEGREE 8 = p+1)
 constexpr int kTreeNodes = 65;    // root + 8x8 children
 constexpr int kGridBuckets = 256;  // of a direction's span lookup grid

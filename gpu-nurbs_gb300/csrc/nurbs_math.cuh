@@ -588,10 +588,18 @@ __device__ __forceinline__ SDer<T> quotient(const RDer<T>& d, T su, T sv) {
 }
 
 // Comparisons of doubles on the integer pipe: an FP64 comparison occupies the FP64 pipe as long as
-// an FP64 multiply-add, a pair of integer instructions a few clocks.  order_key: the order-preserving
-// integer image of a double that is not NaN (-0 and +0 have the same).
+// an FP64 multiply-add, a pair of integer instructions a few clocks.  total_key: the order-preserving
+// integer image of a double that is not NaN, -0 below +0, and key_value its inverse; order_key: the same
+// with one image for -0 and +0, as comparisons see them.
+__device__ __forceinline__ long long total_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double key_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
 __device__ __forceinline__ long long order_key(double x) {
-  const long long b = __double_as_longlong(x), k = b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  const long long k = total_key(x);
   return k == -1 ? 0 : k;
 }
 __device__ __forceinline__ float order_key(float x) { return x; }
