@@ -109,7 +109,10 @@ __global__ void __launch_bounds__(128) k_eval_pool(const SurfDev* __restrict__ t
 }
 
 constexpr int kCtaSpans = 256;      // breakpoint tables staged up to this many spans
-constexpr int kGroupQueries = 128;  // small tiles are taken together up to this many queries
+// Small tiles are taken together up to this many queries.  32 / 64 / 128 / 256, tiles of 16, mixed: 63,000
+// queries of 130 surfaces 1,901 / 1,786 / 1,488 / 1,394 us, 200,000 of 200 4,054 / 3,888 / 4,074 / 4,536; FP64,
+// 63,000 of 130 10,976 / 12,004 / 14,066 / 13,887.
+constexpr int kGroupQueries = 128;
 constexpr int kCtasPerSm = 4;
 
 // Register budget: 4 CTAs per SM (6 / 5 / 4: 6.95 / 6.32 / 6.01 ms on 160 uneven faces in tiles of 128;

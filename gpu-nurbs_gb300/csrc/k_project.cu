@@ -288,9 +288,15 @@ __device__ __forceinline__ int project_polish_step(const Ctx& c, const Eval& ev,
 }
 
 // Slots free or finished before the task list is refilled (invert_core.cuh: a refill culls its new
-// queries and takes the finished ones through the final FP64 steps).
+// queries and takes the finished ones through the final FP64 steps).  16 / 24 / 28 / 30: 2,254 / 2,266 /
+// 2,155 / 2,186 us on 262,147 points of the 64x64 surface, mixed; the same within 2 % on 30,000 and below.
 constexpr int kRefillProj = 28;
-constexpr int kByWarp = 4;  // at the end of a launch, this many running seeds are taken over by the warp
+// At the end of a launch, this many running seeds of a warp are taken over by the whole warp, one after
+// the other.  0 / 2 / 4 / 8: 64x64 surface, mixed, 262,147 points 2,070 / 2,152 / 2,155 / 2,201 us, 500
+// points 146 / 145 / 153 / 171; FP64, 3,000 points 1,576 / 1,196 / 1,385 / 1,653, 20,000 points 1,976 /
+// 1,397 / 1,599 / 1,973; 8x8 surface, FP64, 3,000 points 1,170 / 684 / 1,474 / 1,712; quintic 64x64, FP64,
+// 3,000 points 1,964 / 1,121 / 1,676 / 2,978.
+constexpr int kByWarp = 2;
 
 // One warp projects the queries that `src` hands out, streaming them through its slots as the
 // inversion does (invert_stream).
@@ -673,7 +679,8 @@ cudaError_t launch_project_mode(const SurfDev& s, const double* P_, int64_t n, d
     cached[dev] = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   }
   // at least what puts a warp on every scheduler, up to 16: culling and final steps cost a warp about
-  // as much for one query
+  // as much for one query (8 / 16 / 32: 64x64 surface, FP64, 20,000 points 1,707 / 1,599 / 1,550 us, 8x8
+  // 1,742 / 1,467 / 1,556; mixed the same within 3 %)
   const int64_t spread = n / kSchedulers;
   const int least = (int)(spread < 1 ? 1 : (spread < 16 ? spread : 16));
   int64_t blocks = ((n + least - 1) / least + kWarps - 1) / kWarps;
