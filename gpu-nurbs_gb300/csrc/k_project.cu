@@ -295,8 +295,9 @@ constexpr int kRefillProj = 28;
 // the other.  0 / 2 / 4 / 8: 64x64 surface, mixed, 262,147 points 2,070 / 2,152 / 2,155 / 2,201 us, 500
 // points 146 / 145 / 153 / 171; FP64, 3,000 points 1,576 / 1,196 / 1,385 / 1,653, 20,000 points 1,976 /
 // 1,397 / 1,599 / 1,973; 8x8 surface, FP64, 3,000 points 1,170 / 684 / 1,474 / 1,712; quintic 64x64, FP64,
-// 3,000 points 1,964 / 1,121 / 1,676 / 2,978.
-constexpr int kByWarp = 2;
+// 3,000 points 1,964 / 1,121 / 1,676 / 2,978; 300x40 net, FP64, 6,000 points 2,822 / 1,770 with 2 / 4.  The
+// launch is then as long as one warp's last seeds, so no value is best everywhere; 4 is far off nowhere.
+constexpr int kByWarp = 4;
 
 // One warp projects the queries that `src` hands out, streaming them through its slots as the
 // inversion does (invert_stream).
