@@ -105,21 +105,15 @@ struct Ctx {
   int p, q;
   double dom_u0, dom_u1, dom_v0, dom_v1;
   double iru, irv;   // 1 / knot range
+  bool unit_range;   // both are 1
 };
 
 // |S - P|^2 at (u - du, v - dv) from r = S - P, Su, Sv at (u, v): S(u - du, v - dv) = S - Su du -
 // Sv dv + O(|S''| 1e-20) for the steps a seed ends with (1e-10 at most), below the rounding of S
-// itself.  Su and Sv are scaled by the knot range (kernel.cu:167), so the steps are divided by it.
-// BRANCH: only where it is not 1, for the loops in which some lane ends in nearly every turn (the FP64
-// multiplications are 0.7 % of an FP64 iteration; the branch costs the pool's final steps 1 %).
-template <bool BRANCH>
-__device__ __forceinline__ double dist2_after(const Ctx& c, const v3<double>& r, const v3<double>& Su,
-                                              const v3<double>& Sv, double du, double dv) {
-  const long long one = 0x3ff0000000000000ll;
-  if (!BRANCH || __double_as_longlong(c.iru) != one || __double_as_longlong(c.irv) != one) {
-    du *= c.iru;
-    dv *= c.irv;
-  }
+// itself.  Su and Sv are scaled by the knot range (kernel.cu:167): du and dv are the steps divided by
+// it, or the range is 1.
+__device__ __forceinline__ double dist2_after(const v3<double>& r, const v3<double>& Su, const v3<double>& Sv,
+                                              double du, double dv) {
   const v3<double> r2 = {fast::mad(-Sv.x, dv, fast::mad(-Su.x, du, r.x)),
                          fast::mad(-Sv.y, dv, fast::mad(-Su.y, du, r.y)),
                          fast::mad(-Sv.z, dv, fast::mad(-Su.z, du, r.z))};
@@ -140,6 +134,18 @@ struct GlobalEval {
     return fast::eval_at<float, P, Q, ORDER, true>(c.L32, c.m32, c.p, c.q, u, v, hu, hv);
   }
 };
+
+// The same at an FP64 seed's end (u, v) on a knot range other than 1: evaluated, where the ends are taken
+// up.  (Dividing the steps inside the iterations, in which some lane ends in nearly every turn, cost them
+// up to 2 % on every range.)
+template <int P, int Q>
+__device__ __forceinline__ void evaluate_dist2(const Ctx& c, double px, double py, double pz, double u, double v, int hu,
+                                               int hv, double& dist2) {
+  if (c.unit_range) return;
+  const fast::SDer<double> d = fast::eval_at<double, P, Q, 0>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
+  const v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
+  dist2 = dot3(r, r);
+}
 
 // Per-seed iteration state (hu/hv: span hints for the warm-started span search).
 template <typename T>
@@ -183,7 +189,7 @@ __device__ __forceinline__ int iterate32(const Eval& ev, float px, float py, flo
 
 // One FP64 iteration of a seed (FP64 mode).  dist2, when the seed converges: |S - P|^2 at the new
 // (u, v) from this step's S, Su, Sv (another evaluation for the few lanes whose seeds just ended would
-// cost the warp as much as one for all lanes).
+// cost the warp as much as one for all lanes), for a knot range of 1 (evaluate_dist2).
 template <int P, int Q>
 __device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, double pz, Seed<double>& st,
                                          double& dist2) {
@@ -196,7 +202,7 @@ __device__ __forceinline__ int iterate64(const Ctx& c, double px, double py, dou
   st.v -= dv;
   const double step = fast::max_abs(du, dv);
   if ((st.newton && fast::le_nonneg(step, kTolNewton64)) || fast::le_nonneg(step, kTolAny64)) {
-    dist2 = dist2_after<true>(c, r, d.Su, d.Sv, du, dv);
+    dist2 = dist2_after(r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   st.prev = step;
@@ -295,7 +301,7 @@ __device__ __forceinline__ int final_step(const Ctx& c, const Eval& ev, double p
   f.u -= du;
   f.v -= dv;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewton64)) {
-    const double dist2 = dist2_after<false>(c, r, d.Su, d.Sv, du, dv);
+    const double dist2 = dist2_after(r, d.Su, d.Sv, du * c.iru, dv * c.irv);
     res = sqrt(dist2);
     return in_domain64(c, f.u, f.v, dist2) ? kConverged : kFailed;
   }
@@ -483,7 +489,7 @@ __device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& s
     cx.p = s.p;
     cx.q = s.q;
     cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
-    cx.iru = s.inv_range_u; cx.irv = s.inv_range_v;
+    cx.iru = s.inv_range_u; cx.irv = s.inv_range_v; cx.unit_range = s.unit_range;
   }
 }
 
@@ -931,6 +937,7 @@ __device__ __forceinline__ void invert_stream(Staged<KS, MODE>& sm, WarpWork<MOD
           }
           edge = edge && before(dist, sd.u, sd.v, ww.rec[ql].de, ww.rec[ql].ue, ww.rec[ql].ve);
         } else {
+          if (end == kConverged) evaluate_dist2<P, Q>(cx, tx, ty, tz, sd.u, sd.v, sd.hu, sd.hv, dist);
           upd = end == kConverged && in_domain64(cx, sd.u, sd.v, dist);
           if (upd) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
         }

@@ -38,6 +38,7 @@ __device__ __forceinline__ Ctx global_ctx(const SurfDev& s) {
   cx.dom_v1 = s.dom_v1;
   cx.iru = s.inv_range_u;
   cx.irv = s.inv_range_v;
+  cx.unit_range = s.unit_range;
   return cx;
 }
 
@@ -70,6 +71,7 @@ __device__ bool continue_from(const Ctx& cx, double px, double py, double pz, do
   if (r != kConverged) return false;
   u = sd.u;
   v = sd.v;
+  evaluate_dist2<P, Q>(cx, px, py, pz, u, v, sd.hu, sd.hv, dist2);
   res = sqrt(dist2);
   return in_domain64(cx, u, v, dist2);
 }

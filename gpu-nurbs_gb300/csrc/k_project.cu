@@ -92,10 +92,10 @@ struct PSeed {
 // derivatives are then at hand for its Newton step.  Each trial is evaluated once, with derivatives,
 // and every lane does one evaluation per call: a line search inside the iteration would evaluate the
 // accepted point twice and hold up the warp for its longest search.  dist2: the squared distance, FP32
-// before the last step, FP64 at the end point.
+// before the last step, FP64 at the end point (for a knot range of 1: evaluate_dist2).
 template <typename T>
-__device__ __forceinline__ int project_advance(const Ctx& c, const fast::SDer<T>& d, const T dom[4], T px, T py, T pz,
-                                               PSeed<T>& st, T& dist2) {
+__device__ __forceinline__ int project_advance(const fast::SDer<T>& d, const T dom[4], T px, T py, T pz, PSeed<T>& st,
+                                               T& dist2) {
   constexpr bool kFp32 = sizeof(T) == 4;
   const v3<T> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   const T fn = dot3(r, r);
@@ -175,7 +175,7 @@ __device__ __forceinline__ int project_advance(const Ctx& c, const fast::SDer<T>
   st.trial = false;
   const T du = st.u - st.un, dv = st.v - st.vn;
   if (moved_to()) {
-    if constexpr (!kFp32) dist2 = dist2_after<true>(c, r, d.Su, d.Sv, du, dv);
+    if constexpr (!kFp32) dist2 = dist2_after(r, d.Su, d.Sv, du, dv);
     return kConverged;
   }
   return ++st.it >= kMaxIterProj ? kFailed : kContinue;
@@ -230,7 +230,7 @@ __device__ __forceinline__ int project_by_warp(const Eval& ev, const T dom[4], i
       st.vn = __shfl_sync(FULL, tv, first);
       st.ls = kMaxHalvings;  // taken
     }
-    const int res = project_advance(ev.sm.ctx, ev.template at<2>(st.un, st.vn, hu, hv), dom, px, py, pz, st, dist2);
+    const int res = project_advance(ev.template at<2>(st.un, st.vn, hu, hv), dom, px, py, pz, st, dist2);
     if (res != kContinue) return res;
   }
 }
@@ -280,7 +280,7 @@ __device__ __forceinline__ int project_polish_step(const Ctx& c, const Eval& ev,
   f.u = un;
   f.v = vn;
   if (fast::le_nonneg(fast::max_abs(du, dv), kTolNewtonProj)) {
-    const double dist2 = dist2_after<false>(c, r, d.Su, d.Sv, du, dv);
+    const double dist2 = dist2_after(r, d.Su, d.Sv, du * c.iru, dv * c.irv);
     res = sqrt(dist2);
     return fast::is_finite(dist2) ? kConverged : kFailed;
   }
@@ -296,7 +296,7 @@ constexpr int kRefillProj = 28;
 // points 146 / 145 / 153 / 171; FP64, 3,000 points 1,576 / 1,196 / 1,385 / 1,653, 20,000 points 1,976 /
 // 1,397 / 1,599 / 1,973; 8x8 surface, FP64, 3,000 points 1,170 / 684 / 1,474 / 1,712; quintic 64x64, FP64,
 // 3,000 points 1,964 / 1,121 / 1,676 / 2,978; 300x40 net, FP64, 6,000 points 2,822 / 1,770 with 2 / 4.  The
-// launch is then as long as one warp's last seeds, so no value is best everywhere; 4 is far off nowhere.
+// launch is then as long as one warp's last seeds, and no value is best everywhere.
 constexpr int kByWarp = 4;
 
 // One warp projects the queries that `src` hands out, streaming them through its slots as the
@@ -373,6 +373,7 @@ __device__ __forceinline__ void project_stream(const Staged<kSmemSpans, MODE>& s
           double d2 = 0;
           const int r = project_by_warp(e64, dom64, j, px, py, pz, s64, d2);
           if (lane == j) {
+            if (r == kConverged) evaluate_dist2<P, Q>(cx, px, py, pz, s64.u, s64.v, 0, 0, d2);
             res = r == kConverged && fast::is_finite(d2) ? kConverged : kFailed;
             f.u = s64.u;
             f.v = s64.v;
@@ -586,6 +587,7 @@ __device__ __forceinline__ void project_stream(const Staged<kSmemSpans, MODE>& s
               upd = before(dist, sd.u, sd.v, R.d1, R.u1, R.v1) || before(dist, sd.u, sd.v, R.d2, R.u2, R.v2);
           }
         } else {
+          if (upd) evaluate_dist2<P, Q>(cx, tx, ty, tz, sd.u, sd.v, hu, hv, dist);
           upd = upd && fast::is_finite(dist);
           if (upd) cell_of(sm.cell64, sd.u, sd.v, cu, cv);
         }
@@ -614,7 +616,7 @@ __device__ __forceinline__ void project_stream(const Staged<kSmemSpans, MODE>& s
         }
       }
       if (!waiting) {
-        const int res = project_advance(cx, ev.template at<2>(sd.un, sd.vn, hu, hv), dom, tx, ty, tz, sd, dist);
+        const int res = project_advance(ev.template at<2>(sd.un, sd.vn, hu, hv), dom, tx, ty, tz, sd, dist);
         if (res != kContinue) {
           end = res;
           waiting = true;

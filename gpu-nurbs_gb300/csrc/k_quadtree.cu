@@ -315,7 +315,9 @@ __device__ __noinline__ bool node_trajectory(const SurfDev& s, const SpanTables<
     while (r == kContinue) r = iterate64<P, Q>(cx, px, py, pz, sd, dist2);
     u = sd.u;
     v = sd.v;
-    if (r != kConverged || !in_domain64(cx, u, v, dist2)) return false;
+    if (r != kConverged) return false;
+    evaluate_dist2<P, Q>(cx, px, py, pz, u, v, sd.hu, sd.hv, dist2);
+    if (!in_domain64(cx, u, v, dist2)) return false;
     rr = sqrt(dist2);
     return rr < max_edge;
   }
@@ -642,6 +644,7 @@ __global__ void __launch_bounds__(kThreads, P == 0 ? 2 : 4)
           bool open = false;
           const int k = w.list[slot];
           if (end != kContinue) {
+            if (end == kConverged) evaluate_dist2<P, Q>(cx, tx, ty, tz, sd.u, sd.v, sd.hu, sd.hv, dist);
             const double r = sqrt(dist);
             if (end == kConverged && in_domain64(cx, sd.u, sd.v, dist) && r < max_edge) answer(q0 + k, 0, sd.u, sd.v, r);
             else open = true;

@@ -64,6 +64,7 @@ struct SurfDev {
   int ns_u, ns_v;
   double range_u, range_v;   // k[last]-k[0] (derivative scale numerator, kernel.cu:167-168)
   double inv_range_u, inv_range_v;
+  bool unit_range;           // both ranges are 1
   float range_u32, range_v32;
   double dom_u0, dom_u1, dom_v0, dom_v1;  // knot domain [k[p], k[nu]] x [k[q], k[nv]]
   double org[3];          // origin of the FP32 tables: centre of the control net's bounding box
