@@ -105,7 +105,6 @@ struct Ctx {
   int p, q;
   double dom_u0, dom_u1, dom_v0, dom_v1;
   double iru, irv;   // 1 / knot range
-  bool unit_range;   // both are 1
 };
 
 // |S - P|^2 at (u - du, v - dv) from r = S - P, Su, Sv at (u, v): S(u - du, v - dv) = S - Su du -
@@ -141,7 +140,8 @@ struct GlobalEval {
 template <int P, int Q>
 __device__ __forceinline__ void evaluate_dist2(const Ctx& c, double px, double py, double pz, double u, double v, int hu,
                                                int hv, double& dist2) {
-  if (c.unit_range) return;
+  const long long one = 0x3ff0000000000000ll;
+  if (__double_as_longlong(c.iru) == one && __double_as_longlong(c.irv) == one) return;
   const fast::SDer<double> d = fast::eval_at<double, P, Q, 0>(c.L64, c.m64, c.p, c.q, u, v, hu, hv);
   const v3<double> r = {d.S.x - px, d.S.y - py, d.S.z - pz};
   dist2 = dot3(r, r);
@@ -489,7 +489,7 @@ __device__ __forceinline__ void stage_tables(const SurfDev& s, SpanTables<KS>& s
     cx.p = s.p;
     cx.q = s.q;
     cx.dom_u0 = s.dom_u0; cx.dom_u1 = s.dom_u1; cx.dom_v0 = s.dom_v0; cx.dom_v1 = s.dom_v1;
-    cx.iru = s.inv_range_u; cx.irv = s.inv_range_v; cx.unit_range = s.unit_range;
+    cx.iru = s.inv_range_u; cx.irv = s.inv_range_v;
   }
 }
 

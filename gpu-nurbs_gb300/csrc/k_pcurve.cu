@@ -38,7 +38,6 @@ __device__ __forceinline__ Ctx global_ctx(const SurfDev& s) {
   cx.dom_v1 = s.dom_v1;
   cx.iru = s.inv_range_u;
   cx.irv = s.inv_range_v;
-  cx.unit_range = s.unit_range;
   return cx;
 }
 

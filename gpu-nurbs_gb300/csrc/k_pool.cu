@@ -191,11 +191,11 @@ cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int n
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   if (ctas > ntiles) ctas = ntiles;
-  // (ctas are resident ones: at most pool_ctas_per_sm per SM)
   // Tiles per grab: small tiles together, up to kGroupQueries queries, while every resident CTA gets a
   // grab.  Larger tiles one by one: groups of 8 / 2 / 1 tiles of 128 take 41.3 / 35.8 / 32.8 ms on 600
   // surfaces with 4.4 M queries (the last groups are the launch's tail), and the same on 300 with 1 M.
-  const int group = std::max(1, std::min(ntiles / ctas, kGroupQueries / tile_queries));
+  const int resident = std::min(ctas, kCtasPerSm * 152);
+  const int group = std::max(1, std::min(ntiles / resident, kGroupQueries / tile_queries));
   if (precision == 1)
     k_invert_pool_cta<kModeMixed><<<ctas, kThreads, 0, st>>>(table, tiles, ntiles, counter, P, uv, status, residual,
                                                              group);

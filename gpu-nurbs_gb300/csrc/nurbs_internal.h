@@ -64,7 +64,6 @@ struct SurfDev {
   int ns_u, ns_v;
   double range_u, range_v;   // k[last]-k[0] (derivative scale numerator, kernel.cu:167-168)
   double inv_range_u, inv_range_v;
-  bool unit_range;           // both ranges are 1
   float range_u32, range_v32;
   double dom_u0, dom_u1, dom_v0, dom_v1;  // knot domain [k[p], k[nu]] x [k[q], k[nv]]
   double org[3];          // origin of the FP32 tables: centre of the control net's bounding box
@@ -164,7 +163,6 @@ cudaError_t launch_eval_pool(const SurfDev* table, const InvTile* tiles, int nti
                              unsigned mask, double* out, cudaStream_t st);
 // CTAs of the pool's inversion kernel that an SM of the current GPU holds
 int pool_ctas_per_sm(int precision);
-// ctas: at most what the GPU holds
 cudaError_t launch_invert_pool(const SurfDev* table, const InvTile* tiles, int ntiles, int* counter,
                                const double* P, double* uv, int* status, double* residual, int precision,
                                int ctas, int tile_queries, cudaStream_t st);

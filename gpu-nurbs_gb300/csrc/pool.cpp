@@ -119,7 +119,8 @@ struct nurbs_pool_s {
   std::vector<PoolSurface> surf;
   SurfDev* d_table = nullptr;  // device table of max_surfaces records (outside the arena)
   int tile_queries = 128;
-  int ctas_per_sm = 4;  // launched: this, or as many as an SM holds where that is less (launch_ctas)
+  // launched; an SM holds 4 at once.  160 uneven faces, mixed: 5,434 us with 4, 5,407 with 6
+  int ctas_per_sm = 6;
   int sms = 152;
   std::map<cudaStream_t, Workspace> ws;
   std::set<struct nurbs_graph_s*> graphs;  // live graphs, detached if the pool goes first
@@ -133,11 +134,6 @@ struct nurbs_graph_s {
 };
 
 namespace {
-
-// CTAs of a launch: more than fit at once would start after the others and find the counter exhausted.
-int launch_ctas(nurbs_pool_t P, int ctas_per_sm, int precision) {
-  return P->sms * std::min(ctas_per_sm, pool_ctas_per_sm(precision));
-}
 
 // Tile list of a CSR batch: per surface, ranges of at most tile_q queries; most expensive
 // (higher degree, then larger) tiles first.
@@ -209,7 +205,7 @@ int run_tiles(nurbs_pool_t P, const std::vector<InvTile>& tiles, const double* P
   if (e == cudaSuccess) e = cudaEventRecord(w->ev, st);
   if (e == cudaSuccess)
     e = launch_invert_pool(P->d_table, (const InvTile*)(dev + 256), (int)tiles.size(), (int*)dev, Pd, uv, st_out, res,
-                           precision, launch_ctas(P, ctas_per_sm, precision), tile_q, st);
+                           precision, P->sms * ctas_per_sm, tile_q, st);
   if (e != cudaSuccess) return pfail(NURBS_E_CUDA, "pool inversion: %s", cudaGetErrorString(e));
   return NURBS_OK;
 }
@@ -250,8 +246,8 @@ std::string batch_key(nurbs_pool_t P, int nbatch, const int* ids, const int64_t*
   std::string name = prop.name;
   for (char& ch : name)
     if (ch == ' ') ch = '_';
-  o << name << "/sm" << prop.multiProcessorCount << "/s" << kScheduleVersion << "/prec" << precision << "/n" << nbatch << "/q" << total << "/h"
-    << std::hex << h;
+  o << name << "/sm" << prop.multiProcessorCount << "/s" << kScheduleVersion << "/prec" << precision << "/n" << nbatch
+    << "/q" << total << "/h" << std::hex << h;
   return o.str();
 }
 
@@ -558,7 +554,7 @@ int nurbs_pool_autotune(nurbs_pool_t P, int nbatch, const int* ids, const int64_
   }
   // above 32: throughput; 32 and below: latency, small batches
   const int tile_opts[] = {128, 256, 32, 16};
-  const int fit = pool_ctas_per_sm(precision);  // as many as fit, or fewer for more L1 each
+  const int fit = pool_ctas_per_sm(precision);  // as many as an SM holds, or fewer, with more L1 each
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -630,8 +626,7 @@ int nurbs_pool_graph_create(nurbs_pool_t P, int nbatch, const int* ids, const in
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     cudaError_t le = launch_invert_pool(P->d_table, (const InvTile*)(dev + 256), (int)tiles.size(), (int*)dev, Pd, uv,
-                                        st_out, res, precision, launch_ctas(P, P->ctas_per_sm, precision),
-                                        P->tile_queries, cs);
+                                        st_out, res, precision, P->sms * P->ctas_per_sm, P->tile_queries, cs);
     e = cudaStreamEndCapture(cs, &G->graph);
     if (le != cudaSuccess) e = le;
   }

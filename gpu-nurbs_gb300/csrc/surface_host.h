@@ -187,7 +187,6 @@ inline void fill_surface(const SurfaceHost& S, char* img, char* in_dev, char* ou
   d.range_v = S.kv[S.q + S.nv] - S.kv[0];
   d.inv_range_u = 1.0 / d.range_u;
   d.inv_range_v = 1.0 / d.range_v;
-  d.unit_range = d.range_u == 1.0 && d.range_v == 1.0;
   d.range_u32 = (float)d.range_u;
   d.range_v32 = (float)d.range_v;
   d.dom_u0 = S.ku[S.p]; d.dom_u1 = S.ku[S.nu]; d.dom_v0 = S.kv[S.q]; d.dom_v1 = S.kv[S.nv];

@@ -305,8 +305,8 @@ const char* nurbs_pool_last_error(void);
 /* Launch configuration and persistent CTAs per SM.  tile_queries: queries of one surface
  * that a CTA takes at a time, a multiple of 32 (throughput on large batches) or at most 32 (small
  * batches spread over all SMs; fewer queries per CTA lower latency; large batches take several such
- * tiles at a time).  ctas_per_sm: 1..16; at most as many as an SM holds of the kernel are launched
- * (4 on the GB300, the default). */
+ * tiles at a time).  ctas_per_sm: 1..16, 6 at first; an SM holds 4 at once, more start as others end
+ * and make little difference. */
 int nurbs_pool_set_config(nurbs_pool_t pool, int tile_queries, int ctas_per_sm);
 /* Batched inversion.  Queries are grouped by surface: surface ids_host[k] owns the queries
  * [offsets_host[k], offsets_host[k+1]) of P_dev (3 doubles each); outputs are indexed like P.

@@ -41,7 +41,6 @@ def test_ctas_per_sm(nurbs, work, precision):
     for bad in (0, 17):
         with pytest.raises(nurbs.NurbsError):
             pool.set_config(128, bad)
-    assert nurbs.Pool(1 << 20).info().ctas_per_sm == 4
     assert 1 <= pool.autotune(batch, P, out, precision)[1] <= 4
 
 
