@@ -977,7 +977,7 @@ def serving_record(a, compact=False):
         "config": {"workload": f"serving: pool of {npool} surfaces (batched-workload distribution), 20 GB budget, "
                                "Poisson arrivals, Zipf(1.1) surfaces, 1..4096 queries/request log-uniform, "
                                "10% uploads", "slots": a.slots, "max_batch_queries": a.max_batch_queries,
-                   "queries_per_warp_chunk": a.serve_chunk, "rates_req_s": rates, "seconds_per_rate": serve_seconds},
+                   "tile_queries": a.serve_chunk, "rates_req_s": rates, "seconds_per_rate": serve_seconds},
         "peak": {"req_s": peak["achieved_req_s"], "queries_s": peak["achieved_queries_s"]},
         "half_peak": half, "sweep": sweep,
         "fp64_server_at_top_rate": fp64_peak,
@@ -1071,7 +1071,7 @@ def main():
     ap.add_argument("--slots", type=int, default=4)
     ap.add_argument("--max-batch-queries", type=int, default=1 << 16, help="serving: queries per batch at most")
     ap.add_argument("--upload-frac", type=float, default=0.10)
-    ap.add_argument("--serve-chunk", type=int, default=16, help="queries per warp chunk when serving")
+    ap.add_argument("--serve-chunk", type=int, default=16, help="queries per tile when serving")
     ap.add_argument("--surfaces", type=int, default=4096)
     ap.add_argument("--tune-queries", type=int, default=4 << 20)
     ap.add_argument("--queries", type=int, default=None,

@@ -28,7 +28,7 @@
 //      makes one lane the last.
 //   3. a query whose layer outgrows what a lane keeps is searched on by the whole warp, a node per lane.
 // Measured with a warp per query / a lane per query, its trajectories one after the other / now:
-//   64x64 surface, mixed, 2^18 points within 5e-5      2,585 / 1,557 / 1,181 us  (max_edge 1e-4)
+//   64x64 surface, mixed, 2^18 points within 5e-5      3,236 / 1,548 / 1,270 us  (max_edge 1e-4)
 //   64x64 surface, mixed, 20,000 points off by ~3e-5   1,339 / 3,204 /   729 us  (max_edge 1e-4)
 //   8x8 rough surface, FP64, 20,000 off by ~3e-2       5,172 / 52,467 / 4,103 us (max_edge 0.1: wide layers)
 //   degrees 7 and 4, mixed, 6,000 off by ~3e-3         3,457 / 6,963 / 2,156 us  (max_edge 1e-2)
